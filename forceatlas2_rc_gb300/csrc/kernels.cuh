@@ -56,6 +56,14 @@ __device__ __forceinline__ typename RT<R>::R4 mk4(R a, R b, R c, R d)
     return v;
 }
 
+// d^2 of the tree's walks: one fixed contraction in float, so that every walk
+// makes the same decisions and sums the same terms; none in double.
+__device__ __forceinline__ float sq_dist(float xd, float yd)
+{
+    return __fmaf_rn(xd, xd, __fmul_rn(yd, yd));
+}
+__device__ __forceinline__ double sq_dist(double xd, double yd) { return xd * xd + yd * yd; }
+
 // Repulsion factor between two nodes (reference src/forceatlas2.c:265-275,
 // pipeline.cl:46-55): the force on the first is (xd, yd) * factor.
 template <class R, bool ADJUST>
@@ -470,8 +478,12 @@ __device__ __forceinline__ float4 agg_record(const Agg<float> &q, float wscale)
 {
     const float m = q.m.hi + q.m.lo;
     const float w = q.maxx - q.minx, h = q.maxy - q.miny;
-    return make_float4(__fdiv_rn(q.mx.hi + q.mx.lo, m), __fdiv_rn(q.my.hi + q.my.lo, m), m,
-                       2.0f * (w * w + h * h) * wscale);
+    // the rounded centre kept inside the box: a region of coincident nodes (w
+    // = h = 0) has its centre exactly at its nodes, which are then not far
+    // from it
+    const float cx = fminf(fmaxf(__fdiv_rn(q.mx.hi + q.mx.lo, m), q.minx), q.maxx);
+    const float cy = fminf(fmaxf(__fdiv_rn(q.my.hi + q.my.lo, m), q.miny), q.maxy);
+    return make_float4(cx, cy, m, 2.0f * (w * w + h * h) * wscale);
 }
 
 // Arrival at region r: returns the number of children that arrived before
@@ -743,7 +755,7 @@ walk(int k, int n, R scaling, R theta2, double theta2d,
             if (j != k) {
                 const R4 q = psort[j];
                 const R xd = xi - q.x, yd = yi - q.y;
-                const R g = rep_factor<R, ADJUST>(xd * xd + yd * yd, mi * q.z,
+                const R g = rep_factor<R, ADJUST>(sq_dist(xd, yd), mi * q.z,
                                                   si + q.w, scaling);
                 ax += xd * g;
                 ay += yd * g;
@@ -763,7 +775,7 @@ walk(int k, int n, R scaling, R theta2, double theta2d,
         const R4 c = rec_c[cur];
         const int2 t = rec_t[cur];
         const R xd = xi - c.x, yd = yi - c.y;
-        const R d2 = xd * xd + yd * yd;
+        const R d2 = sq_dist(xd, yd);
         const bool far = region_far(d2, c.w, theta2, agg + cur, (float) xi, (float) yi, theta2d);
         if (far) {
             const R g = fdiv(scaling * (mi * c.z), d2);
@@ -849,7 +861,7 @@ __device__ __forceinline__ void sum_pairs(int k, const int *q, int nq, R xi, R y
         if (j != k) {
             const typename RT<R>::R4 p = ldg_r4(psort + j);
             const R xd = xi - p.x, yd = yi - p.y;
-            const R g = rep_factor<R, ADJUST>(xd * xd + yd * yd, mi * p.z, si + p.w, scaling);
+            const R g = rep_factor<R, ADJUST>(sq_dist(xd, yd), mi * p.z, si + p.w, scaling);
             acc_add(ax, cx, xd * g, comp);
             acc_add(ay, cy, yd * g, comp);
         }
@@ -899,7 +911,7 @@ walk_deferred(int k, int n, R scaling, R theta2, double theta2d,
             const R4 c = ldg_r4(rec_c + cur);
             const int2 t = __ldg(rec_t + cur);
             const R xd = xi - c.x, yd = yi - c.y;
-            const R d2 = xd * xd + yd * yd;
+            const R d2 = sq_dist(xd, yd);
             const bool far =
                 region_far(d2, c.w, theta2, agg + cur, (float) xi, (float) yi, theta2d);
             if (far) {
@@ -995,7 +1007,7 @@ walk_multi(int k0, int cnt, int n, R scaling, R theta2, double theta2d,
             for (int u = 0; u < P; u++) {
                 if (((pairs >> u) & 1u) && j != k0 + u) {
                     const R xd = xi[u] - q.x, yd = yi[u] - q.y;
-                    const R g = rep_factor<R, ADJUST>(xd * xd + yd * yd, mi[u] * q.z,
+                    const R g = rep_factor<R, ADJUST>(sq_dist(xd, yd), mi[u] * q.z,
                                                       si[u] + q.w, scaling);
                     ax[u] += xd * g;
                     ay[u] += yd * g;
@@ -1024,7 +1036,7 @@ walk_multi(int k0, int cnt, int n, R scaling, R theta2, double theta2d,
         for (int u = 0; u < P; u++) {
             if (!((act >> u) & 1u)) continue;
             const R xd = xi[u] - c.x, yd = yi[u] - c.y;
-            const R d2 = xd * xd + yd * yd;
+            const R d2 = sq_dist(xd, yd);
             const bool far =
                 region_far(d2, c.w, theta2, agg + cur, (float) xi[u], (float) yi[u], theta2d);
             if (far) {
@@ -1109,7 +1121,7 @@ k_traverse_warp(int n, R scaling, R theta2, double theta2d,
             if (j >= resume && j != k) {
                 const R4 q = psort[j];
                 const R xd = xi - q.x, yd = yi - q.y;
-                const R g = rep_factor<R, ADJUST>(xd * xd + yd * yd, mi * q.z, si + q.w,
+                const R g = rep_factor<R, ADJUST>(sq_dist(xd, yd), mi * q.z, si + q.w,
                                                   scaling);
                 ax += xd * g;
                 ay += yd * g;
@@ -1123,7 +1135,7 @@ k_traverse_warp(int n, R scaling, R theta2, double theta2d,
         bool open = false, direct = false;
         if (rg.x >= resume) {
             const R xd = xi - c.x, yd = yi - c.y;
-            const R d2 = xd * xd + yd * yd;
+            const R d2 = sq_dist(xd, yd);
             const bool far =
                 region_far(d2, c.w, theta2, agg + cur, (float) xi, (float) yi, theta2d);
             if (far) {
@@ -1143,7 +1155,7 @@ k_traverse_warp(int n, R scaling, R theta2, double theta2d,
                 const R4 q = psort[j];
                 if (direct && j != k) {
                     const R xd = xi - q.x, yd = yi - q.y;
-                    const R g = rep_factor<R, ADJUST>(xd * xd + yd * yd, mi * q.z, si + q.w,
+                    const R g = rep_factor<R, ADJUST>(sq_dist(xd, yd), mi * q.z, si + q.w,
                                                       scaling);
                     ax += xd * g;
                     ay += yd * g;
@@ -1180,7 +1192,7 @@ k_traverse_count(int n, R theta2, double theta2d, const typename RT<R>::R4 *__re
             const typename RT<R>::R4 c = rec_c[cur];
             const int2 t = rec_t[cur];
             const R xd = me.x - c.x, yd = me.y - c.y;
-            const R d2 = xd * xd + yd * yd;
+            const R d2 = sq_dist(xd, yd);
             const bool far =
                 region_far(d2, c.w, theta2, agg + cur, (float) me.x, (float) me.y, theta2d);
             if (far) {
