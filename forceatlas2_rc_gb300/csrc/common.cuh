@@ -23,11 +23,13 @@ void set_cuda_error(const char *what, cudaError_t e);
         }                                                                      \
     } while (0)
 
-// Barnes-Hut walk variants (all give identical forces): warp-synchronous;
-// one walk per thread at 8 blocks of 256 per SM (<= 32 registers; 6 and <= 40
-// with prevent_overlap or in double); one walk
-// per thread with the registers the compiler wants; one thread walking for
-// two or four Morton neighbours at once.
+// Barnes-Hut walk variants (the same interactions; all but the last give
+// identical forces): warp-synchronous; one walk per thread at 8 blocks of 256
+// per SM (<= 32 registers; 6 and <= 40 with prevent_overlap or in double);
+// one walk per thread with the registers the compiler wants; one thread
+// walking for two or four Morton neighbours at once; the node pairs summed
+// after the regions (float: a warp's 32 nodes together, group_walk.cuh;
+// double: one walk per thread).
 enum {
     WALK_WARP = 0,
     WALK_THREAD = 1,

@@ -812,7 +812,8 @@ k_traverse(int n, R scaling, R theta2, double theta2d,
                                   rope, status);
 }
 
-// The walk with its node pairs deferred (FP32 path). In the walk above, a
+// The walk with its node pairs deferred (the batched FP32 layouts). In the
+// walk above, a
 // warp whose lanes are partly summing node pairs and partly visiting
 // regions issues both kinds of step in nearly every iteration. Here the walk
 // visits regions only: a small region that is too close (and a single node
@@ -955,11 +956,42 @@ k_traverse_deferred(int n, R scaling, R theta2, double theta2d,
                     const uint32_t *__restrict__ order, typename RT<R>::R2 *__restrict__ f,
                     int *__restrict__ status)
 {
-    pdl_wait();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     f[order[k]] = walk_deferred<R, ADJUST, COMP>(k, n, scaling, theta2, theta2d, psort, rec_c,
                                                  rec_t, agg, rope, status);
+}
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p)
+{
+    return (uint32_t) __cvta_generic_to_shared(p);
+}
+
+} // namespace fa2cu
+
+#include "group_walk.cuh"
+
+namespace fa2cu {
+
+// The group walk (group_walk.cuh) of every node, a warp's 32 neighbours
+// together; `split` warps (1, 2 or 4) share the walk of 32 nodes.
+constexpr int GW_WARPS = 4;
+template <bool ADJUST, bool HUBS>
+__global__ void __launch_bounds__(32 * GW_WARPS, 9)
+k_traverse_group(int n, int split, float scaling, double theta2d, const float4 *__restrict__ psort,
+                 const float4 *__restrict__ rec_c, const int2 *__restrict__ rec_t,
+                 const int2 *__restrict__ child, const Agg<float> *__restrict__ agg,
+                 const uint32_t *__restrict__ order, float2 *__restrict__ f,
+                 int *__restrict__ status)
+{
+    __shared__ GroupTopShared T;
+    __shared__ GroupWalkShared S[GW_WARPS];
+    pdl_wait();
+    const int base0 = blockIdx.x * (32 * GW_WARPS / split);
+    const float2 v = group_walk_block<ADJUST, HUBS>(T, S, base0, split, n, scaling, theta2d, psort,
+                                                    rec_c, rec_t, child, agg, status);
+    const int w = threadIdx.x >> 5, k = base0 + 32 * (w / split) + (int) (threadIdx.x & 31);
+    if (w % split == 0 && k < n) f[order[k]] = v;
 }
 
 // The walk of P sorted nodes k0 .. k0+cnt-1 (cnt <= P, neighbours in
@@ -1907,11 +1939,6 @@ k_forces_out(int n, const typename RT<R>::R2 *__restrict__ f, const int *__restr
 template <class R> __host__ __device__ constexpr int exact_tile()
 {
     return 8192 / (int) sizeof(typename RT<R>::R4);
-}
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p)
-{
-    return (uint32_t) __cvta_generic_to_shared(p);
 }
 
 

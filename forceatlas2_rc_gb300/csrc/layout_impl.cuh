@@ -66,10 +66,23 @@ template <class R> struct Layout : LayoutBase {
 
     int n = 0, ninc = 0, repulsion = 0, adjust = 0, strong = 0, linlog = 0;
     int any_fixed = 0;
-    // FP32: the walk with deferred node pairs (0.48-0.52 against 0.57-0.61
-    // ms at 10^6 nodes); FP64: one walk per thread, in the reference's
-    // order of the forces
+    // FP32: the group walk (group_walk.cuh); FP64: one walk per thread, in
+    // the reference's order of the forces
     int walk = sizeof(R) == 4 ? WALK_DEFERRED : WALK_THREAD;
+    // Warps that share the group walk of 32 nodes, from the warps the device
+    // holds at once (36 an SM, 5472 in all): a layout too small to fill it is
+    // bound by the serial chain of one warp's rounds, which more warps
+    // shorten; a full device by the instructions, of which each part repeats
+    // the first rounds. The repulsion in us with 1 / 2 / 4 warps: 3,001 nodes
+    // 31.7 / 25.2 / 22.9; 10,007 35.6 / 27.2 / 24.6; 30,011 (radii) 40.8 /
+    // 32.4 / 30.3; 50,007 45.5 / 37.7 / 44.9; 100,000 57.4 / 63.7 / 79.7;
+    // 300,007 118 / 158 / 236.
+    int walk_split = 1;
+    static int pick_split(int n)
+    {
+        const double x = n / 32.0 / 5472.0; // of the device, with one warp each
+        return x < 0.22 ? 4 : x < 0.45 ? 2 : 1;
+    }
     int climb_mode = 1; // leaves per aggregate thread (negative: interleaved)
     bool block_sort = false; // few keys: the one-block sort
 
@@ -327,6 +340,7 @@ template <class R> struct Layout : LayoutBase {
         if (rep == FA2CU_REPULSION_BH && sort_setup()) return 1;
         if (rep == FA2CU_REPULSION_BH) {
             climb_mode = pick_climb(n, device);
+            walk_split = pick_split(n);
             // sort tiles: fewer than ~75 tiles of 8192 keys leave most SMs
             // idle; measured on a GB300 (sort of one iteration, ms, tiles of
             // 256 / 512 / 1024 threads): 1e5 keys 0.050 / 0.051 / 0.060;
@@ -495,6 +509,18 @@ template <class R> struct Layout : LayoutBase {
                      child, parent, range, rope, visits, agg, rec_c, rec_t, wscale, status);
         }
     }
+    // (graphs with hubs: their walks add up with compensation)
+    void launch_group_walk()
+    {
+        auto go = [&](auto kernel) {
+            launch_k(pdl, kernel, dim3(ceil_div(n, 32 * GW_WARPS / walk_split)),
+                     dim3(32 * GW_WARPS), 0, s, n, walk_split, scaling, theta2d, psort, rec_c, rec_t, child, agg, order, f, status);
+        };
+        if (adjust)
+            nheavy > 0 ? go(k_traverse_group<true, true>) : go(k_traverse_group<true, false>);
+        else
+            nheavy > 0 ? go(k_traverse_group<false, true>) : go(k_traverse_group<false, false>);
+    }
     void launch_repulsion()
     {
         if (repulsion == FA2CU_REPULSION_BH) {
@@ -517,27 +543,18 @@ template <class R> struct Layout : LayoutBase {
                                                           rec_c, rec_t, agg, rope, order, f,
                                                           status);
             } else if (walk == WALK_DEFERRED) {
-                // graphs with hubs: their walks add up with compensation
-                const int g = ceil_div(n, 256);
-                // (every deferred walk waits for its predecessor first)
-                if (adjust) {
-                    if (nheavy > 0)
-                        launch_k(pdl, k_traverse_deferred<R, true, 6, true>, dim3(g), dim3(256),
-                                 0, s, n, scaling, theta2, theta2d, psort, rec_c, rec_t, agg,
-                                 rope, order, f, status);
-                    else
-                        launch_k(pdl, k_traverse_deferred<R, true, 6>, dim3(g), dim3(256), 0, s,
-                                 n, scaling, theta2, theta2d, psort, rec_c, rec_t, agg, rope,
-                                 order, f, status);
+                if constexpr (sizeof(R) == 4) {
+                    launch_group_walk();
                 } else {
-                    if (nheavy > 0)
-                        launch_k(pdl, k_traverse_deferred<R, false, sizeof(R) == 4 ? 8 : 6, true>,
-                                 dim3(g), dim3(256), 0, s, n, scaling, theta2, theta2d, psort,
-                                 rec_c, rec_t, agg, rope, order, f, status);
+                    const int g = ceil_div(n, 256);
+                    if (adjust)
+                        k_traverse_deferred<R, true, 6><<<g, 256, 0, s>>>(
+                            n, scaling, theta2, theta2d, psort, rec_c, rec_t, agg, rope, order,
+                            f, status);
                     else
-                        launch_k(pdl, k_traverse_deferred<R, false, sizeof(R) == 4 ? 8 : 6>,
-                                 dim3(g), dim3(256), 0, s, n, scaling, theta2, theta2d, psort,
-                                 rec_c, rec_t, agg, rope, order, f, status);
+                        k_traverse_deferred<R, false, 6><<<g, 256, 0, s>>>(
+                            n, scaling, theta2, theta2d, psort, rec_c, rec_t, agg, rope, order,
+                            f, status);
                 }
             } else if (walk == WALK_PAIR) {
                 const int grid = ceil_div(ceil_div(n, 2), 256);
@@ -886,6 +903,10 @@ template <class R> struct Layout : LayoutBase {
 
     int option(const char *name, double value) override
     {
+        if (!strcmp(name, "walk_split") && (value == 1 || value == 2 || value == 4)) {
+            walk_split = (int) value;
+            return recapture();
+        }
         if (!strcmp(name, "sort_threads") && (value == 256 || value == 512 || value == 1024)) {
             ss.tile_threads = (int) value;
             return recapture();

@@ -86,10 +86,13 @@ int fa2cu_layout_traversal_counts(fa2cu_layout *L, double counts[2]);
  *                  (default in double precision), 0 warp-synchronous (lanes
  *                  walk together, keeping their own decisions), 2 the
  *                  per-thread walk compiled without its register bound, 3 /
- *                  4 two / four Morton neighbours per thread, 5 one walk per
- *                  thread visiting regions only, its node pairs queued and
- *                  summed after the far regions (default in single
- *                  precision);
+ *                  4 two / four Morton neighbours per thread, 5 the regions
+ *                  first, the node pairs queued and summed after them
+ *                  (default in single precision, where a warp walks for 32
+ *                  Morton neighbours together);
+ *   "walk_split"   single precision: warps that share the walk of 32 nodes,
+ *                  1, 2 or 4 (default: 4 below 38,000 nodes, 2 below
+ *                  79,000, else 1; forces equal to ~1e-7);
  *   "climb"        leaves per thread of the bottom-up sums: 1, 2, 4 or 8
  *                  contiguous, -2 or -4 interleaved over the warp (default:
  *                  1 below one wave of threads, else 2 in float, 4 in
