@@ -1630,12 +1630,16 @@ __device__ __forceinline__ void swing_finish(SwingAcc<R> acc, int n, const uint8
             str[i] = skip ? R(0) : __ldcg(tr + i);
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
+        // one lane sums the swinging, another the traction: an add of a
+        // warp's two lanes costs what one lane's does (64 cycles a dependent
+        // FP64 add)
+        if (threadIdx.x < 2) {
+            const R *v = threadIdx.x == 0 ? ssw : str;
+            double s = 0.0;
 #pragma unroll 8
-            for (int i = 0; i < n; i++) {
-                tsw = __dadd_rn(tsw, (double) ssw[i]);
-                ttr = __dadd_rn(ttr, (double) str[i]);
-            }
+            for (int i = 0; i < n; i++) s = __dadd_rn(s, (double) v[i]);
+            tsw = s;
+            ttr = __shfl_down_sync(3u, s, 1);
         }
     } else if constexpr (sizeof(R) == 4) {
         // the partials per thread (strided, fixed order) and per warp in
@@ -2108,6 +2112,79 @@ k_exact(int n, R scaling, const typename RT<R>::R4 *__restrict__ nodes,
                 f[i] = mk2<R>(ax[u], ay[u]);
         }
     }
+}
+
+// The all-pairs sum in double with the pairs of a few nodes spread over a
+// block: its producer threads compute the terms of a tile of sources, two
+// pairs each, and one warp adds them up, a lane per node and coordinate, in
+// ascending order of the source -- the terms of k_exact's one thread per node,
+// added in the same order, hence the same bits. The adds (64 cycles each,
+// dependent) of a tile run while the next tile's terms are computed.
+//
+// Bound: the FP64 pipe, about 21 operations a pair at 2 lanes a cycle and SM,
+// and 16 cycles a source for the adds of up to 16 nodes. Against one thread
+// per node, 256 a block (1,500 nodes kept 6 of the 152 SMs busy), in us: 150
+// nodes 222 -> 18, 1,500 2138 -> 134, 6,007 8569 -> 1574, 20,000 28,530 ->
+// 15,838, 40,000 113,641 -> 62,042.
+constexpr int EXACT_ORDERED_PAIRS = 1024; // of a tile, two per producer
+constexpr int EXACT_ORDERED_ROWS = 16;    // nodes a block at most
+constexpr int EXACT_ORDERED_THREADS = EXACT_ORDERED_PAIRS / 2 + 32;
+template <bool ADJUST>
+__global__ void __launch_bounds__(EXACT_ORDERED_THREADS)
+k_exact_ordered(int n, int rows, double scaling, const double4_32a *__restrict__ nodes,
+                double2 *__restrict__ f)
+{
+    constexpr int PAIRS = EXACT_ORDERED_PAIRS;
+    // the nodes' rows one element apart in bank: [buffer][coordinate]
+    __shared__ double term[2][2][PAIRS + EXACT_ORDERED_ROWS];
+    const int tile = PAIRS / rows, stride = tile + 1; // sources a tile
+    const int row0 = blockIdx.x * rows;
+    const int ntiles = (n + tile - 1) / tile;
+    const bool adder = threadIdx.x >= PAIRS / 2;
+    const int lane = threadIdx.x & 31;
+    double sum = 0.0;
+    // a producer's two pairs: fixed nodes, sources a tile apart each time
+    int at[2], src[2];
+    double4_32a me[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int q = threadIdx.x + h * (PAIRS / 2), r = q / tile;
+        src[h] = !adder && r < rows && row0 + r < n ? q % tile : n;
+        at[h] = r * stride + q % tile;
+        me[h] = nodes[min(row0 + r, n - 1)];
+    }
+    for (int t = 0; t <= ntiles; t++) {
+        if (!adder) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                if (src[h] < n) {
+                    const double4_32a p = nodes[src[h]];
+                    const double xd = me[h].x - p.x, yd = me[h].y - p.y;
+                    const double g = rep_factor<double, ADJUST>(
+                        xd * xd + yd * yd, me[h].z * p.z, me[h].w + p.w, scaling);
+                    term[t & 1][0][at[h]] = xd * g;
+                    term[t & 1][1][at[h]] = yd * g;
+                    src[h] += tile;
+                }
+            }
+        } else if (t > 0 && lane < 2 * rows) {
+            const double *q = &term[(t - 1) & 1][lane & 1][(lane >> 1) * stride];
+            const int cnt = min(tile, n - (t - 1) * tile);
+#pragma unroll 8
+            for (int j = 0; j < cnt; j++) sum = __dadd_rn(sum, q[j]);
+        }
+        __syncthreads();
+    }
+    const int i = row0 + (lane >> 1);
+    if (adder && lane < 2 * rows && i < n) reinterpret_cast<double *>(f + i)[lane & 1] = sum;
+}
+
+// Nodes a block of k_exact_ordered: the fewest blocks an SM that keep to
+// EXACT_ORDERED_ROWS, with the blocks even over the SMs.
+inline int exact_ordered_rows(int n, int sms)
+{
+    const int per_sm = (n + sms * EXACT_ORDERED_ROWS - 1) / (sms * EXACT_ORDERED_ROWS);
+    return (n + sms * per_sm - 1) / (sms * per_sm);
 }
 
 // The rows of k_exact's partial sums, in row order.

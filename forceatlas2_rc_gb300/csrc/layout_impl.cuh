@@ -38,6 +38,15 @@ inline double now_s()
     return (double) ts.tv_sec + 1e-9 * (double) ts.tv_nsec;
 }
 
+// SMs of the current device (at least 1).
+inline int device_sms()
+{
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return std::max(sms, 1);
+}
+
 // The all-pairs repulsion of n packed records into f: k_exact over `rows`
 // source ranges (exact_rows), then their fixed-order sum when rows > 1
 // (partial holds rows * n entries).
@@ -45,19 +54,44 @@ template <class R, int IPT>
 void launch_exact(cudaStream_t s, int n, bool adjust, R scaling, const typename RT<R>::R4 *packed,
                   typename RT<R>::R2 *f, typename RT<R>::R2 *partial, int rows, int *status)
 {
-    constexpr int TILE = exact_tile<R>();
-    const int seg = rows > 1 ? ceil_div(ceil_div(n, rows), TILE) * TILE : ceil_div(n, TILE) * TILE;
-    rows = ceil_div(n, seg);
-    const dim3 grid(ceil_div(n, FA2_EXACT_THREADS * IPT), rows);
-    const size_t smem = exact_smem_bytes<R>();
-    typename RT<R>::R2 *part = rows > 1 ? partial : nullptr;
-    if (adjust)
-        k_exact<R, true, IPT><<<grid, FA2_EXACT_THREADS, smem, s>>>(n, scaling, packed, f, part,
-                                                                    seg, status);
-    else
-        k_exact<R, false, IPT><<<grid, FA2_EXACT_THREADS, smem, s>>>(n, scaling, packed, f, part,
-                                                                     seg, status);
-    if (rows > 1) k_exact_sum<R><<<ceil_div(n, 256), 256, 0, s>>>(n, rows, partial, f);
+    if constexpr (sizeof(R) == 8) {
+        const int per = exact_ordered_rows(n, device_sms()), grid = ceil_div(n, per);
+        if (adjust)
+            k_exact_ordered<true><<<grid, EXACT_ORDERED_THREADS, 0, s>>>(n, per, scaling, packed, f);
+        else
+            k_exact_ordered<false><<<grid, EXACT_ORDERED_THREADS, 0, s>>>(n, per, scaling, packed,
+                                                                          f);
+    } else {
+        constexpr int TILE = exact_tile<R>();
+        const int seg =
+            rows > 1 ? ceil_div(ceil_div(n, rows), TILE) * TILE : ceil_div(n, TILE) * TILE;
+        rows = ceil_div(n, seg);
+        const dim3 grid(ceil_div(n, FA2_EXACT_THREADS * IPT), rows);
+        const size_t smem = exact_smem_bytes<R>();
+        typename RT<R>::R2 *part = rows > 1 ? partial : nullptr;
+        if (adjust)
+            k_exact<R, true, IPT><<<grid, FA2_EXACT_THREADS, smem, s>>>(n, scaling, packed, f,
+                                                                        part, seg, status);
+        else
+            k_exact<R, false, IPT><<<grid, FA2_EXACT_THREADS, smem, s>>>(n, scaling, packed, f,
+                                                                         part, seg, status);
+        if (rows > 1) k_exact_sum<R><<<ceil_div(n, 256), 256, 0, s>>>(n, rows, partial, f);
+    }
+}
+
+// The dynamic shared memory of the all-pairs kernel, on the current device.
+template <class R, int IPT> int setup_exact()
+{
+    if constexpr (sizeof(R) == 4) {
+        const int smem = (int) exact_smem_bytes<R>();
+        FA2_TRY(cudaFuncSetAttribute(k_exact<R, false, IPT>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+                "cudaFuncSetAttribute", 1);
+        FA2_TRY(cudaFuncSetAttribute(k_exact<R, true, IPT>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+                "cudaFuncSetAttribute", 1);
+    }
+    return 0;
 }
 
 template <class R> struct Layout : LayoutBase {
@@ -427,13 +461,7 @@ template <class R> struct Layout : LayoutBase {
         h.n = n;
         FA2_TRY(cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, s), "cudaMemcpy", 1);
         if (repulsion == FA2CU_REPULSION_EXACT) {
-            const size_t smem = exact_smem_bytes<R>();
-            FA2_TRY(cudaFuncSetAttribute(k_exact<R, false, EXACT_IPT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
-                    "cudaFuncSetAttribute", 1);
-            FA2_TRY(cudaFuncSetAttribute(k_exact<R, true, EXACT_IPT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
-                    "cudaFuncSetAttribute", 1);
+            if (setup_exact<R, EXACT_IPT>()) return 1;
         }
         FA2_TRY(cudaStreamSynchronize(s), "could not prepare the layout", 1);
         if (capture(&g1, 1)) return 1;
@@ -1116,13 +1144,7 @@ template <class R> struct Repulse : RepulseBase {
         FA2_TRY(cudaMallocHost(&host2, 2 * nn * sizeof(double)), "out of memory", 1);
         FA2_TRY(cudaMemsetAsync(status, 0, ST_COUNT * sizeof(int), s), "cudaMemset", 1);
         if (!barnes_hut) {
-            const size_t smem = exact_smem_bytes<R>();
-            FA2_TRY(cudaFuncSetAttribute(k_exact<R, false, Layout<R>::EXACT_IPT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
-                    "cudaFuncSetAttribute", 1);
-            FA2_TRY(cudaFuncSetAttribute(k_exact<R, true, Layout<R>::EXACT_IPT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem),
-                    "cudaFuncSetAttribute", 1);
+            if (setup_exact<R, Layout<R>::EXACT_IPT>()) return 1;
         }
         FA2_TRY(cudaStreamSynchronize(s), "could not prepare the device", 1);
         return 0;
