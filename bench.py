@@ -531,7 +531,7 @@ def run_exact(args):
     pairs = float(n) * n
     tflops = 20.0 * pairs / (ms / 1000.0) / 1e12
     print(json.dumps({"workload": f"exact all-pairs repulsion, n={n}, FP32",
-                      "kernel": "k_exact<float, 0, 4> (+ k_pack, k_exact_sum)",
+                      "kernel": "k_exact<0, 6>",
                       "launch_ms": ms,
                       "pairs_per_s": pairs / (ms / 1000.0),
                       "fp32_tflops_20flop_convention": tflops,

@@ -56,6 +56,38 @@ __device__ __forceinline__ typename RT<R>::R4 mk4(R a, R b, R c, R d)
     return v;
 }
 
+// A source as the all-pairs kernels read it. FP32: two coordinates and the
+// mass and radius, each twice, side by side, so that one packed (f32x2)
+// instruction combines a source with two nodes; the coordinates negated, so
+// that a difference is one addition. FP64: (x, y, m, r).
+struct alignas(32) ExactF32 {
+    float nx[2], ny[2], m[2], r[2];
+};
+template <class R> struct ExactRec;
+template <> struct ExactRec<float> {
+    typedef ExactF32 type;
+};
+template <> struct ExactRec<double> {
+    typedef double4_32a type;
+};
+__device__ __forceinline__ void exact_move(ExactF32 *e, float2 p)
+{
+    *reinterpret_cast<float4 *>(e) = make_float4(-p.x, -p.x, -p.y, -p.y);
+}
+__device__ __forceinline__ void exact_move(double4_32a *e, double2 p)
+{
+    *reinterpret_cast<double2 *>(e) = p;
+}
+__device__ __forceinline__ void exact_fill(ExactF32 *e, float2 p, float m, float r)
+{
+    exact_move(e, p);
+    reinterpret_cast<float4 *>(e)[1] = make_float4(m, m, r, r);
+}
+__device__ __forceinline__ void exact_fill(double4_32a *e, double2 p, double m, double r)
+{
+    *e = mk4<double>(p.x, p.y, m, r);
+}
+
 // d^2 of the tree's walks: one fixed contraction in float, so that every walk
 // makes the same decisions and sums the same terms; none in double.
 __device__ __forceinline__ float sq_dist(float xd, float yd)
@@ -1248,6 +1280,30 @@ k_traverse_count(int n, R theta2, double theta2d, const typename RT<R>::R4 *__re
 
 // ---- 6. gravity and attraction (pipeline.cl:389-429) -----------------------
 
+// Node i's all-pairs repulsion: the rows of the partial sums, in row order.
+template <class R>
+__device__ __forceinline__ typename RT<R>::R2
+exact_sum(int i, int n, int rows, const typename RT<R>::R2 *partial)
+{
+    typedef typename RT<R>::R2 R2;
+    R2 a = partial[i];
+    // (a row's entry a load: eight in flight)
+    constexpr int U = 8;
+    for (int r0 = 1; r0 < rows; r0 += U) {
+        R2 b[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (r0 + u < rows) b[u] = partial[(size_t) (r0 + u) * n + i];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (r0 + u < rows) {
+                a.x += b[u].x;
+                a.y += b[u].y;
+            }
+    }
+    return a;
+}
+
 // Nodes of at least this many incidences (hubs of scale-free graphs) are
 // summed by a warp each in the FP32 path (k_attract_heavy, launched before
 // the attraction): one thread looping over a hub's thousands of incidences
@@ -1714,8 +1770,8 @@ __device__ __forceinline__ void swing_finish(SwingAcc<R> acc, int n, const uint8
 // launch for the attraction and the totals.
 template <class R>
 __global__ void __launch_bounds__(256)
-k_attract_swing(int n, R gravity, int strong, int linlog, int adjust,
-                const typename RT<R>::R2 *__restrict__ pos, const R *__restrict__ mass,
+k_attract_swing(int n, R gravity, int strong, int linlog, int adjust, int rows,
+                const typename RT<R>::R2 *__restrict__ partial_f, const typename RT<R>::R2 *__restrict__ pos, const R *__restrict__ mass,
                 const R *__restrict__ size, const int *__restrict__ off,
                 const Inc<R> *__restrict__ inc, typename RT<R>::R2 *__restrict__ f,
                 const typename RT<R>::R2 *__restrict__ fold, const uint8_t *__restrict__ fixed,
@@ -1723,9 +1779,12 @@ k_attract_swing(int n, R gravity, int strong, int linlog, int adjust,
                 unsigned *__restrict__ ticket, SpeedState *__restrict__ st,
                 int *__restrict__ status)
 {
+    pdl_wait();
     SwingAcc<R> acc;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
+        // the all-pairs repulsion still in rows (not yet in f)
+        if (rows > 0) f[i] = exact_sum<R>(i, n, rows, partial_f);
         attract_one<R, sizeof(R) == 4>(i, gravity, strong, linlog, adjust, pos, mass, size, off,
                                        inc, f);
         swing_node<R>(i, n, f, fold, mass, fixed, sw, tr, acc);
@@ -1804,7 +1863,7 @@ k_apply(int n, int adjust, const typename RT<R>::R2 *__restrict__ f,
         const uint8_t *__restrict__ fixed, typename RT<R>::R2 *__restrict__ pos,
         const SpeedState *__restrict__ st, const int *__restrict__ status,
         R *__restrict__ partial, R *__restrict__ bbox, double *__restrict__ quant,
-        unsigned *__restrict__ ticket)
+        unsigned *__restrict__ ticket, typename ExactRec<R>::type *__restrict__ rec)
 {
     pdl_wait();
     const bool stopped = status[ST_ERROR] != 0;
@@ -1831,6 +1890,7 @@ k_apply(int n, int adjust, const typename RT<R>::R2 *__restrict__ f,
                 p.x += a.x * factor;
                 p.y += a.y * factor;
                 pos[i] = p;
+                if (rec) exact_move(rec + i, p); // the all-pairs kernel's record
             }
         }
         mnx = cl_min(mnx, p.x);
@@ -1884,21 +1944,8 @@ k_inc_in(int ninc, const int *__restrict__ node, const double *__restrict__ coef
     inc[e] = c;
 }
 
-// (x, y, m, r) records of every node in original order (the exact kernel's
-// input); r = 0 unless adjust.
-template <class R>
-__global__ void __launch_bounds__(256)
-k_pack(int n, int adjust, const typename RT<R>::R2 *__restrict__ pos,
-       const R *__restrict__ mass, const R *__restrict__ size,
-       typename RT<R>::R4 *__restrict__ out)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const typename RT<R>::R2 p = pos[i];
-    out[i] = mk4<R>(p.x, p.y, mass[i], adjust ? size[i] : R(0));
-}
-
-// Same records from four host-layout double arrays (fa2_gpu_repulse_*).
+// (x, y, m, r) records from four host-layout double arrays
+// (fa2_gpu_repulse_bh).
 template <class R>
 __global__ void __launch_bounds__(256)
 k_pack_host(int n, const double *__restrict__ x, const double *__restrict__ y,
@@ -1926,25 +1973,44 @@ k_forces_out(int n, const typename RT<R>::R2 *__restrict__ f, const int *__restr
 }
 
 // ---- exact repulsion: the n-body tile kernel ------------------------------
-// Each thread owns IPT nodes (i, i + T, ...) and sums over every j in
-// ascending order, as the reference (src/forceatlas2.c:278-294). Tiles of
-// (x, y, m, r) records are staged in shared memory by TMA bulk copies
-// (cp.async.bulk, completion on an mbarrier), two tiles in flight. The pair
-// i == j contributes exactly zero (xd = yd = 0 with a finite factor), so no
-// test is needed. Every mbarrier wait is bounded in time: on expiry the
-// kernel records ERR_WAIT, drains its copies in flight and returns.
-
-#define FA2_EXACT_THREADS 256
-#ifndef FA2_EXACT_IPT_F32
-#define FA2_EXACT_IPT_F32 4 // nodes per thread in FP32 (FP64: 1)
-#endif
-
-// Records per tile of the all-pairs kernel (8 KB of records, double-buffered).
-template <class R> __host__ __device__ constexpr int exact_tile()
+// Records of every node in original order; r = 0 unless adjust.
+template <class R>
+__global__ void __launch_bounds__(256)
+k_pack(int n, int adjust, const typename RT<R>::R2 *__restrict__ pos,
+       const R *__restrict__ mass, const R *__restrict__ size,
+       typename ExactRec<R>::type *__restrict__ out)
 {
-    return 8192 / (int) sizeof(typename RT<R>::R4);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) exact_fill(out + i, pos[i], mass[i], adjust ? size[i] : R(0));
 }
 
+// The same from four host-layout double arrays (fa2_gpu_repulse_exact).
+template <class R>
+__global__ void __launch_bounds__(256)
+k_pack_exact(int n, const double *__restrict__ x, const double *__restrict__ y,
+             const double *__restrict__ m, const double *__restrict__ s,
+             typename ExactRec<R>::type *__restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n)
+        exact_fill(out + i, mk2<R>((R) x[i], (R) y[i]), (R) m[i], s ? (R) s[i] : R(0));
+}
+
+// FP32. Each thread owns IPT nodes (i, i + T, ...), two to a packed
+// instruction, and sums over its range of sources in ascending order. Tiles
+// of records are staged in shared memory by TMA bulk copies (cp.async.bulk,
+// completion on an mbarrier), two tiles in flight. The pair i == j
+// contributes exactly zero (xd = yd = 0 with a finite factor), so no test is
+// needed. Every mbarrier wait is bounded in time: on expiry the kernel
+// records ERR_WAIT, drains its copies in flight and returns.
+//
+// Bound: the FP32 pipe, 7 operations a pair (and one MUFU reciprocal, at half
+// their time); the packed instructions leave its issue slots for the rest.
+// 100,003 nodes: 2906 -> 2426 us (77 % of the pipe at 2070 MHz; with 4 nodes a
+// thread 2568, with 8 2525, with 10 2471).
+
+constexpr int EXACT_THREADS = 256;
+constexpr int EXACT_TILE = 256; // records (8 KB, double-buffered)
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count)
 {
@@ -1990,39 +2056,40 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned phase,
     }
 }
 
-// Block (x, y) sums, for its FA2_EXACT_THREADS * IPT nodes, the sources
-// [y seg, min(n, (y + 1) seg)) (seg a multiple of the tile): into f when the
-// grid has one row (every j, ascending: the reference's order), else into
-// row y of `partial` (n entries per row), summed by k_exact_sum.
-template <class R, bool ADJUST, int IPT>
-__global__ void __launch_bounds__(FA2_EXACT_THREADS)
-k_exact(int n, R scaling, const typename RT<R>::R4 *__restrict__ nodes,
-        typename RT<R>::R2 *__restrict__ f, typename RT<R>::R2 *__restrict__ partial, int seg,
-        int *__restrict__ status)
+// Block (x, y) sums, for its EXACT_THREADS * IPT nodes, the sources [y seg,
+// min(n, (y + 1) seg)) into row y of `partial` (n entries a row); the rows are
+// added in order by who reads them (exact_sum).
+template <bool ADJUST, int IPT>
+__global__ void __launch_bounds__(EXACT_THREADS)
+k_exact(int n, float scaling, const ExactF32 *__restrict__ nodes, float2 *__restrict__ partial,
+        int seg, int *__restrict__ status)
 {
-    typedef typename RT<R>::R4 R4;
-    constexpr int TILE = exact_tile<R>();
-    extern __shared__ __align__(128) unsigned char smem[];
-    R4 *tile = reinterpret_cast<R4 *>(smem);
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem + 2 * TILE * sizeof(R4));
+    static_assert(IPT % 2 == 0, "two nodes to a packed instruction");
+    constexpr int P = IPT / 2;
+    __shared__ __align__(128) ExactF32 tile[2][EXACT_TILE];
+    __shared__ uint64_t bar[2];
     __shared__ int failed;
+    pdl_wait();
 
-    R xi[IPT], yi[IPT], mi[IPT], si[IPT], smi[IPT], ax[IPT], ay[IPT];
-    const int i0 = blockIdx.x * (FA2_EXACT_THREADS * IPT) + threadIdx.x;
+    GroupNode me[P];
+    float mi[IPT], si[IPT];
+    f2 ax[P], ay[P];
+    const int i0 = blockIdx.x * (EXACT_THREADS * IPT) + threadIdx.x;
 #pragma unroll
-    for (int u = 0; u < IPT; u++) {
-        const int i = i0 + u * FA2_EXACT_THREADS;
-        const R4 p = nodes[i < n ? i : n - 1];
-        xi[u] = p.x;
-        yi[u] = p.y;
-        mi[u] = p.z;
-        si[u] = p.w;
-        smi[u] = scaling * p.z;
-        ax[u] = ay[u] = R(0);
+    for (int u = 0; u < P; u++) {
+        const int a = min(i0 + 2 * u * EXACT_THREADS, n - 1);
+        const int b = min(i0 + (2 * u + 1) * EXACT_THREADS, n - 1);
+        me[u].x = f2_make(-nodes[a].nx[0], -nodes[b].nx[0]);
+        me[u].y = f2_make(-nodes[a].ny[0], -nodes[b].ny[0]);
+        mi[2 * u] = scaling * nodes[a].m[0];
+        mi[2 * u + 1] = scaling * nodes[b].m[0];
+        si[2 * u] = nodes[a].r[0];
+        si[2 * u + 1] = nodes[b].r[0];
+        ax[u] = ay[u] = 0;
     }
     const int j0 = blockIdx.y * seg, j1 = min(n, j0 + seg);
-    const R4 *src = nodes + j0;
-    const int ntiles = (j1 - j0 + TILE - 1) / TILE;
+    const ExactF32 *src = nodes + j0;
+    const int ntiles = (j1 - j0 + EXACT_TILE - 1) / EXACT_TILE;
     if (threadIdx.x == 0) {
         failed = 0;
         mbar_init(&bar[0], 1);
@@ -2033,11 +2100,12 @@ k_exact(int n, R scaling, const typename RT<R>::R4 *__restrict__ nodes,
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int t = 0; t < 2 && t < ntiles; t++) {
-            const int cnt = min(TILE, j1 - j0 - t * TILE);
-            tma_load_1d(tile + t * TILE, src + (size_t) t * TILE, cnt * (unsigned) sizeof(R4),
-                        &bar[t]);
+            const int cnt = min(EXACT_TILE, j1 - j0 - t * EXACT_TILE);
+            tma_load_1d(tile[t], src + (size_t) t * EXACT_TILE,
+                        cnt * (unsigned) sizeof(ExactF32), &bar[t]);
         }
     }
+    const f2 tiny = f2_make(1e-30f, 1e-30f);
     for (int t = 0; t < ntiles; t++) {
         const int b = t & 1;
         if (!mbar_wait(&bar[b], (t >> 1) & 1, 2000000000ull)) failed = 1;
@@ -2052,65 +2120,61 @@ k_exact(int n, R scaling, const typename RT<R>::R4 *__restrict__ nodes,
             __syncthreads();
             return;
         }
-        const R4 *q = tile + b * TILE;
-        const int cnt = min(TILE, j1 - j0 - t * TILE);
-        if constexpr (sizeof(R) == 4 && !ADJUST) {
-            // FP32: 7 FP32-pipe operations and one MUFU reciprocal per
-            // pair; the thread's scaling * m_i multiplies the sums once at
-            // the end. d2 carries 1e-30 (d2 = xd^2 + (yd^2 + 1e-30), one FMA
-            // each): a coincident pair (xd = yd = 0) then has a finite
-            // factor below 1e30 * m_j, so its term is 0 -- the reference's
-            // factor for d2 = 0 -- without a compare; any other pair of
-            // float positions is at least ~1e-14 apart in d2 for
-            // coordinates of 1e-3 or more, which the 1e-30 leaves unchanged
-            // to float precision.
+        const int cnt = min(EXACT_TILE, j1 - j0 - t * EXACT_TILE);
+        unsigned q = smem_addr(tile[b]);
+        // d2 carries 1e-30 (d2 = xd^2 + (yd^2 + 1e-30), one FMA each): a
+        // coincident pair (xd = yd = 0) then has a finite factor below 1e30
+        // m_j, so its term is 0 -- the reference's factor for d2 = 0 --
+        // without a compare; any other pair of float positions is at least
+        // ~1e-14 apart in d2 for coordinates of 1e-3 or more, which the 1e-30
+        // leaves unchanged to float precision. The thread's scaling * m_i
+        // multiplies the sums once at the end.
 #pragma unroll 4
-            for (int jj = 0; jj < cnt; jj++) {
-                const R4 p = q[jj];
+        for (int jj = 0; jj < cnt; jj++, q += (unsigned) sizeof(ExactF32)) {
+            f2 nx, ny, m, r;
+            lds_2<0>(q, nx, ny);
+            if (ADJUST)
+                lds_2<16>(q, m, r);
+            else
+                m = lds_1<16>(q);
 #pragma unroll
-                for (int u = 0; u < IPT; u++) {
-                    const float xd = xi[u] - p.x, yd = yi[u] - p.y;
-                    const float d2 = fmaf(xd, xd, fmaf(yd, yd, 1e-30f));
-                    const float g = p.z * __fdividef(1.0f, d2);
-                    ax[u] = fmaf(xd, g, ax[u]);
-                    ay[u] = fmaf(yd, g, ay[u]);
+            for (int u = 0; u < P; u++) {
+                const f2 xd = f2_add(me[u].x, nx), yd = f2_add(me[u].y, ny);
+                f2 g;
+                if (ADJUST) {
+                    float d2a, d2b, ma, mb, ra, rb;
+                    f2_split(f2_fma(xd, xd, f2_mul(yd, yd)), d2a, d2b);
+                    f2_split(m, ma, mb);
+                    f2_split(r, ra, rb);
+                    const float da = fsqrt(d2a) - (si[2 * u] + ra);
+                    const float db = fsqrt(d2b) - (si[2 * u + 1] + rb);
+                    g = f2_make(
+                        da > 0.0f ? ma * rcp_approx(da * da) : da < 0.0f ? 100.0f * ma : 0.0f,
+                        db > 0.0f ? mb * rcp_approx(db * db) : db < 0.0f ? 100.0f * mb : 0.0f);
+                } else {
+                    g = pull2(m, f2_fma(xd, xd, f2_fma(yd, yd, tiny)));
                 }
-            }
-        } else {
-#pragma unroll 4
-            for (int jj = 0; jj < cnt; jj++) {
-                const R4 p = q[jj];
-#pragma unroll
-                for (int u = 0; u < IPT; u++) {
-                    const R xd = xi[u] - p.x, yd = yi[u] - p.y;
-                    const R g = rep_factor<R, ADJUST>(xd * xd + yd * yd, mi[u] * p.z,
-                                                      si[u] + p.w, scaling);
-                    ax[u] += xd * g;
-                    ay[u] += yd * g;
-                }
+                ax[u] = f2_fma(xd, g, ax[u]);
+                ay[u] = f2_fma(yd, g, ay[u]);
             }
         }
         __syncthreads(); // every thread is done with buffer b
         if (threadIdx.x == 0 && t + 2 < ntiles) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            const int cnt2 = min(TILE, j1 - j0 - (t + 2) * TILE);
-            tma_load_1d(tile + b * TILE, src + (size_t) (t + 2) * TILE,
-                        cnt2 * (unsigned) sizeof(R4), &bar[b]);
+            const int cnt2 = min(EXACT_TILE, j1 - j0 - (t + 2) * EXACT_TILE);
+            tma_load_1d(tile[b], src + (size_t) (t + 2) * EXACT_TILE,
+                        cnt2 * (unsigned) sizeof(ExactF32), &bar[b]);
         }
     }
+    float2 *row = partial + (size_t) blockIdx.y * n;
 #pragma unroll
-    for (int u = 0; u < IPT; u++) {
-        const int i = i0 + u * FA2_EXACT_THREADS;
-        if (sizeof(R) == 4 && !ADJUST) {
-            ax[u] *= smi[u];
-            ay[u] *= smi[u];
-        }
-        if (i < n) {
-            if (partial)
-                partial[(size_t) blockIdx.y * n + i] = mk2<R>(ax[u], ay[u]);
-            else
-                f[i] = mk2<R>(ax[u], ay[u]);
-        }
+    for (int u = 0; u < P; u++) {
+        const int a = i0 + 2 * u * EXACT_THREADS, b = a + EXACT_THREADS;
+        float xa, xb, ya, yb;
+        f2_split(ax[u], xa, xb);
+        f2_split(ay[u], ya, yb);
+        if (a < n) row[a] = make_float2(xa * mi[2 * u], ya * mi[2 * u]);
+        if (b < n) row[b] = make_float2(xb * mi[2 * u + 1], yb * mi[2 * u + 1]);
     }
 }
 
@@ -2187,43 +2251,27 @@ inline int exact_ordered_rows(int n, int sms)
     return (n + sms * per_sm - 1) / (sms * per_sm);
 }
 
-// The rows of k_exact's partial sums, in row order.
 template <class R>
 __global__ void __launch_bounds__(256)
 k_exact_sum(int n, int rows, const typename RT<R>::R2 *__restrict__ partial,
             typename RT<R>::R2 *__restrict__ f)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    typename RT<R>::R2 a = partial[i];
-    for (int r = 1; r < rows; r++) {
-        const typename RT<R>::R2 b = partial[(size_t) r * n + i];
-        a.x += b.x;
-        a.y += b.y;
-    }
-    f[i] = a;
+    if (i < n) f[i] = exact_sum<R>(i, n, rows, partial);
 }
 
-template <class R> constexpr size_t exact_smem_bytes()
+// Source ranges (rows) of an n-node FP32 all-pairs sum on a GPU of `sms` SMs,
+// of at least 16 sources each: two blocks an SM for small layouts, whose rows
+// the attraction adds up (an iteration in us with 2 / 4 / 8 blocks an SM:
+// 2,000 nodes 19.8 / 22.4 / 22.4; 6,007 30.4 / 32.4 / 37.4; 9,999 48.0 / 48.3 /
+// 50.0), the eight an SM holds for large ones (20,000 133.9 / 126.9 / 124.5;
+// 40,000 516 / 451 / 437; 100,003 - / 2699 / 2591).
+inline int exact_rows(int n, int sms, int ipt)
 {
-    return 2 * (size_t) exact_tile<R>() * sizeof(typename RT<R>::R4) + 2 * sizeof(uint64_t);
+    const int nb = (n + EXACT_THREADS * ipt - 1) / (EXACT_THREADS * ipt);
+    const int rows = std::min((n < 12000 ? 2 : 8) * sms / nb, n / 16);
+    return std::max(1, rows);
 }
-
-// Rows of source ranges for an n-node all-pairs sum on a GPU of `sms` SMs:
-// enough blocks for about six per SM, each range at least two tiles long;
-// 1 in double (every node sums every j in order) or when n alone fills the
-// GPU.
-template <class R> int exact_rows(int n, int sms, int ipt)
-{
-    if (sizeof(R) != 4) return 1;
-    const int nb = (n + FA2_EXACT_THREADS * ipt - 1) / (FA2_EXACT_THREADS * ipt);
-    const int want = (6 * sms + nb - 1) / nb;
-    const int most = n / (2 * exact_tile<R>());
-    int rows = want < most ? want : most;
-    if (rows > 16) rows = 16;
-    return rows < 1 ? 1 : rows;
-}
-
 
 // ---- quadtree traversal of fa2_gpu_repulse_bh (reference src/gpu.c:78-123)
 // Regions of the host's Gephi quadtree, converted on the device.

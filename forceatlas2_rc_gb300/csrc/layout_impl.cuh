@@ -47,12 +47,18 @@ inline int device_sms()
     return std::max(sms, 1);
 }
 
-// The all-pairs repulsion of n packed records into f: k_exact over `rows`
-// source ranges (exact_rows), then their fixed-order sum when rows > 1
-// (partial holds rows * n entries).
-template <class R, int IPT>
-void launch_exact(cudaStream_t s, int n, bool adjust, R scaling, const typename RT<R>::R4 *packed,
-                  typename RT<R>::R2 *f, typename RT<R>::R2 *partial, int rows, int *status)
+// FP32 nodes a thread of the all-pairs kernel: six share a source's loads;
+// with few nodes two, for more threads (4,000 nodes: 23 against 28 us an
+// iteration).
+inline int exact_ipt(int n) { return n < 4096 ? 2 : 6; }
+
+// The all-pairs repulsion of n records. FP32: `rows` rows of partial sums
+// (n entries each; exact_rows) into `partial`, for exact_sum to add up -- or,
+// one row, straight into f. FP64: into f.
+template <class R>
+void launch_exact(cudaStream_t s, bool pdl, int n, bool adjust, R scaling,
+                  const typename ExactRec<R>::type *packed, typename RT<R>::R2 *f,
+                  typename RT<R>::R2 *partial, int rows, int *status)
 {
     if constexpr (sizeof(R) == 8) {
         const int per = exact_ordered_rows(n, device_sms()), grid = ceil_div(n, per);
@@ -62,36 +68,17 @@ void launch_exact(cudaStream_t s, int n, bool adjust, R scaling, const typename 
             k_exact_ordered<false><<<grid, EXACT_ORDERED_THREADS, 0, s>>>(n, per, scaling, packed,
                                                                           f);
     } else {
-        constexpr int TILE = exact_tile<R>();
-        const int seg =
-            rows > 1 ? ceil_div(ceil_div(n, rows), TILE) * TILE : ceil_div(n, TILE) * TILE;
-        rows = ceil_div(n, seg);
-        const dim3 grid(ceil_div(n, FA2_EXACT_THREADS * IPT), rows);
-        const size_t smem = exact_smem_bytes<R>();
-        typename RT<R>::R2 *part = rows > 1 ? partial : nullptr;
+        const int seg = ceil_div(n, rows), ipt = exact_ipt(n);
+        auto go = [&](auto kernel) {
+            launch_k(pdl, kernel, dim3(ceil_div(n, EXACT_THREADS * ipt), rows),
+                     dim3(EXACT_THREADS), 0, s, n, scaling, packed, rows > 1 ? partial : f, seg,
+                     status);
+        };
         if (adjust)
-            k_exact<R, true, IPT><<<grid, FA2_EXACT_THREADS, smem, s>>>(n, scaling, packed, f,
-                                                                        part, seg, status);
+            ipt == 2 ? go(k_exact<true, 2>) : go(k_exact<true, 6>);
         else
-            k_exact<R, false, IPT><<<grid, FA2_EXACT_THREADS, smem, s>>>(n, scaling, packed, f,
-                                                                         part, seg, status);
-        if (rows > 1) k_exact_sum<R><<<ceil_div(n, 256), 256, 0, s>>>(n, rows, partial, f);
+            ipt == 2 ? go(k_exact<false, 2>) : go(k_exact<false, 6>);
     }
-}
-
-// The dynamic shared memory of the all-pairs kernel, on the current device.
-template <class R, int IPT> int setup_exact()
-{
-    if constexpr (sizeof(R) == 4) {
-        const int smem = (int) exact_smem_bytes<R>();
-        FA2_TRY(cudaFuncSetAttribute(k_exact<R, false, IPT>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-                "cudaFuncSetAttribute", 1);
-        FA2_TRY(cudaFuncSetAttribute(k_exact<R, true, IPT>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-                "cudaFuncSetAttribute", 1);
-    }
-    return 0;
 }
 
 template <class R> struct Layout : LayoutBase {
@@ -169,8 +156,9 @@ template <class R> struct Layout : LayoutBase {
     int nbbox = 1;
     uint32_t *key = nullptr, *order = nullptr;
     SortScratch ss{};
-    R4 *psort = nullptr, *packed = nullptr;
-    R2 *exact_part = nullptr; // exact_rows rows of partial sums (rows > 1)
+    R4 *psort = nullptr;
+    typename ExactRec<R>::type *packed = nullptr; // exact repulsion: the nodes' records
+    R2 *exact_part = nullptr; // exact_rows rows of partial sums (FP32, rows > 1)
     int exact_nrows = 1;
     int2 *child = nullptr, *range = nullptr;
     int *parent = nullptr, *rope = nullptr, *visits = nullptr;
@@ -263,7 +251,7 @@ template <class R> struct Layout : LayoutBase {
             rec_t = mem.get<int2>(nn - 1);
             if (sizeof(R) == 4) fatt = mem.get<R2>(nn);
         } else {
-            packed = mem.get<R4>(nn);
+            packed = mem.get<typename ExactRec<R>::type>(nn);
             if (exact_nrows > 1) exact_part = mem.get<R2>((size_t) exact_nrows * nn);
         }
         if (mem.failed) {
@@ -388,7 +376,8 @@ template <class R> struct Layout : LayoutBase {
         if (rep == FA2CU_REPULSION_EXACT) {
             int sms = 0;
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-            exact_nrows = exact_rows<R>(n, std::max(sms, 1), EXACT_IPT);
+            exact_nrows = exact_layout_rows(n, sms);
+            pdl = n < 500000;
         }
         if (alloc(rep == FA2CU_REPULSION_BH)) return 1;
 
@@ -460,16 +449,18 @@ template <class R> struct Layout : LayoutBase {
         h.jitter_tolerance = p->jitter_tolerance;
         h.n = n;
         FA2_TRY(cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, s), "cudaMemcpy", 1);
-        if (repulsion == FA2CU_REPULSION_EXACT) {
-            if (setup_exact<R, EXACT_IPT>()) return 1;
-        }
         FA2_TRY(cudaStreamSynchronize(s), "could not prepare the layout", 1);
         if (capture(&g1, 1)) return 1;
         if (n <= (1 << 16) && capture(&g8, 8)) return 1;
         return 0;
     }
 
-    static constexpr int EXACT_IPT = sizeof(R) == 4 ? FA2_EXACT_IPT_F32 : 1;
+    static int exact_layout_rows(int n, int sms)
+    {
+        if (sizeof(R) == 8) return 1;
+        const int rows = exact_rows(n, std::max(sms, 1), exact_ipt(n));
+        return ceil_div(n, ceil_div(n, rows)); // (no empty row)
+    }
 
     // ---- the steps of one iteration ----
     // The bounding box and Morton quantisation of the current positions (the
@@ -609,10 +600,15 @@ template <class R> struct Layout : LayoutBase {
                         n, scaling, theta2, theta2d, psort, rec_c, rec_t, agg, rope, order, f, status);
             }
         } else {
-            k_pack<R><<<ceil_div(n, 256), 256, 0, s>>>(n, adjust, pos, mass, size, packed);
-            launch_exact<R, EXACT_IPT>(s, n, adjust, scaling, packed, f, exact_part, exact_nrows,
-                                       status);
+            launch_exact<R>(s, pdl, n, adjust, scaling, packed, f, exact_part, exact_nrows,
+                            status);
         }
+    }
+    // The all-pairs repulsion into f, where it is still in rows.
+    void launch_exact_sum()
+    {
+        if (repulsion == FA2CU_REPULSION_EXACT && exact_nrows > 1)
+            k_exact_sum<R><<<ceil_div(n, 256), 256, 0, s>>>(n, exact_nrows, exact_part, f);
     }
     // The heavy nodes' attraction (FP32), added to their repulsion.
     void launch_heavy()
@@ -624,6 +620,7 @@ template <class R> struct Layout : LayoutBase {
     // Attraction and gravity only (the forces of fa2cu_layout_forces).
     void launch_attraction()
     {
+        launch_exact_sum();
         launch_heavy();
         k_attract<R><<<ceil_div(n, 256), 256, 0, s>>>(n, gravity, strong, linlog, adjust, pos,
                                                       mass, size, inc_off, inc, f);
@@ -634,10 +631,16 @@ template <class R> struct Layout : LayoutBase {
     {
         // serial totals: the last block stages 2n reals
         const size_t smem = serial_totals<R>(n) ? 2 * (size_t) n * sizeof(R) : 0;
+        // the rows of the all-pairs sum are added up in the same launch,
+        // unless a hub's attraction is added to them first
+        const bool in_rows =
+            repulsion == FA2CU_REPULSION_EXACT && exact_nrows > 1 && nheavy == 0;
+        if (!in_rows) launch_exact_sum();
         launch_heavy();
-        k_attract_swing<R><<<ceil_div(n, 256), 256, smem, s>>>(
-            n, gravity, strong, linlog, adjust, pos, mass, size, inc_off, inc, f, fold, fixed, sw,
-            trac, swing_partial, (unsigned *) (status + ST_TICKET_SWING), st, status);
+        launch_k(pdl && nheavy == 0, k_attract_swing<R>, dim3(ceil_div(n, 256)), dim3(256), smem,
+                 s, n, gravity, strong, linlog, adjust, in_rows ? exact_nrows : 0, exact_part,
+                 pos, mass, size, inc_off, inc, f, fold, fixed, sw, trac, swing_partial,
+                 (unsigned *) (status + ST_TICKET_SWING), st, status);
     }
     // The displacement, with the next iteration's bounding box.
     void launch_move()
@@ -646,7 +649,8 @@ template <class R> struct Layout : LayoutBase {
         // one thread per node
         const int nb = bbox_partial ? nbbox : ceil_div(n, 256);
         launch_k(pdl, k_apply<R>, dim3(nb), dim3(256), 0, s, n, adjust, f, fold, sw, fixed, pos,
-                 st, status, bbox_partial, bbox, quant, (unsigned *) (status + ST_TICKET_BBOX));
+                 st, status, bbox_partial, bbox, quant, (unsigned *) (status + ST_TICKET_BBOX),
+                 packed);
     }
     void launch_repel()
     {
@@ -808,6 +812,8 @@ template <class R> struct Layout : LayoutBase {
                 "could not send the positions to the device", 1);
         k_pos_in<R><<<ceil_div(n, 256), 256, 0, s>>>(n, xy, pos);
         if (bbox_partial) launch_bbox();
+        if (packed) // (the displacement keeps them up to date)
+            k_pack<R><<<ceil_div(n, 256), 256, 0, s>>>(n, adjust, pos, mass, size, packed);
         FA2_TRY(cudaStreamSynchronize(s), "could not send the positions to the device", 1);
         return 0;
     }
@@ -1078,7 +1084,7 @@ double layout_footprint(int n, int ninc, int adjust, int any_fixed, int rep, int
     L.adjust = adjust ? 1 : 0;
     L.any_fixed = any_fixed ? 1 : 0;
     if (rep == FA2CU_REPULSION_EXACT)
-        L.exact_nrows = exact_rows<R>(n, std::max(sms, 1), Layout<R>::EXACT_IPT);
+        L.exact_nrows = Layout<R>::exact_layout_rows(n, sms);
     L.mem.dry = true;
     L.alloc(rep == FA2CU_REPULSION_BH);
     const double staging = (double) std::max(n, ninc) * sizeof(double) + (double) ninc * sizeof(int);
@@ -1096,7 +1102,8 @@ template <class R> struct Repulse : RepulseBase {
     double *in4 = nullptr;   // x, y, mass, size staging (4n)
     double *out2 = nullptr;  // fx, fy (2n)
     double *host2 = nullptr; // pinned copy of out2
-    R4 *p = nullptr;
+    R4 *p = nullptr;                         // Barnes-Hut records, tree order
+    typename ExactRec<R>::type *e = nullptr; // all-pairs records
     R2 *f = nullptr;
     R2 *part = nullptr; // partial sums of the split all-pairs kernel
     int nrows = 1;
@@ -1123,16 +1130,11 @@ template <class R> struct Repulse : RepulseBase {
                 "could not create a CUDA stream", 1);
         in4 = mem.get<double>(4 * nn);
         out2 = mem.get<double>(2 * nn);
-        p = mem.get<R4>(nn);
         f = mem.get<R2>(nn);
         status = mem.get<int>(ST_COUNT);
-        if (!barnes_hut) {
-            int sms = 0;
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-            nrows = exact_rows<R>(n, std::max(sms, 1), Layout<R>::EXACT_IPT);
-            if (nrows > 1) part = mem.get<R2>((size_t) nrows * nn);
-        }
+        if (!barnes_hut) get_exact();
         if (barnes_hut) {
+            p = mem.get<R4>(nn);
             raw = mem.get<fa2_region>(2 * nn);
             regs = mem.get<QRegion<R>>(2 * nn);
             perm = mem.get<int>(nn);
@@ -1143,14 +1145,21 @@ template <class R> struct Repulse : RepulseBase {
         }
         FA2_TRY(cudaMallocHost(&host2, 2 * nn * sizeof(double)), "out of memory", 1);
         FA2_TRY(cudaMemsetAsync(status, 0, ST_COUNT * sizeof(int), s), "cudaMemset", 1);
-        if (!barnes_hut) {
-            if (setup_exact<R, Layout<R>::EXACT_IPT>()) return 1;
-        }
         FA2_TRY(cudaStreamSynchronize(s), "could not prepare the device", 1);
         return 0;
     }
 
-    int send4(const double *x, const double *y, const double *m, const double *sz)
+    // The buffers of the all-pairs repulsion (in a Barnes-Hut session, on its
+    // first use).
+    void get_exact()
+    {
+        if (e) return;
+        e = mem.get<typename ExactRec<R>::type>((size_t) n);
+        nrows = Layout<R>::exact_layout_rows(n, device_sms());
+        if (nrows > 1) part = mem.get<R2>((size_t) nrows * n);
+    }
+
+    int send4(const double *x, const double *y, const double *m, const double *sz, bool all_pairs)
     {
         const size_t b = (size_t) n * sizeof(double);
         FA2_TRY(cudaMemcpyAsync(in4, x, b, cudaMemcpyHostToDevice, s), "the computation on the GPU failed", 1);
@@ -1160,8 +1169,13 @@ template <class R> struct Repulse : RepulseBase {
         if (with_size)
             FA2_TRY(cudaMemcpyAsync(in4 + 3 * (size_t) n, sz, b, cudaMemcpyHostToDevice, s),
                     "the computation on the GPU failed", 1);
-        k_pack_host<R><<<ceil_div(n, 256), 256, 0, s>>>(
-            n, in4, in4 + n, in4 + 2 * (size_t) n, with_size ? in4 + 3 * (size_t) n : nullptr, p);
+        const double *dsz = with_size ? in4 + 3 * (size_t) n : nullptr;
+        if (all_pairs)
+            k_pack_exact<R><<<ceil_div(n, 256), 256, 0, s>>>(n, in4, in4 + n,
+                                                             in4 + 2 * (size_t) n, dsz, e);
+        else
+            k_pack_host<R><<<ceil_div(n, 256), 256, 0, s>>>(n, in4, in4 + n,
+                                                            in4 + 2 * (size_t) n, dsz, p);
         return 0;
     }
 
@@ -1198,12 +1212,18 @@ template <class R> struct Repulse : RepulseBase {
               double sc, double *dx, double *dy) override
     {
         cudaSetDevice(device);
+        get_exact();
+        if (mem.failed) {
+            set_cuda_error("could not allocate memory on the device", mem.err);
+            return 1;
+        }
         double t0 = now_s();
-        if (send4(x, y, m, sz)) return 1;
+        if (send4(x, y, m, sz, true)) return 1;
         FA2_TRY(cudaStreamSynchronize(s), "the computation on the GPU failed", 1);
         double t1 = now_s();
         t_send += t1 - t0;
-        launch_exact<R, Layout<R>::EXACT_IPT>(s, n, adjust, (R) sc, p, f, part, nrows, status);
+        launch_exact<R>(s, false, n, adjust, (R) sc, e, f, part, nrows, status);
+        if (nrows > 1) k_exact_sum<R><<<ceil_div(n, 256), 256, 0, s>>>(n, nrows, part, f);
         FA2_TRY(cudaGetLastError(), "the computation on the GPU failed", 1);
         FA2_TRY(cudaStreamSynchronize(s), "the computation on the GPU failed", 1);
         if (check_status()) return 1;
@@ -1216,7 +1236,7 @@ template <class R> struct Repulse : RepulseBase {
         cudaSetDevice(device);
         if (check_quadtree(n, t)) return 1;
         double t0 = now_s();
-        if (send4(t->px, t->py, t->pm, t->ps)) return 1;
+        if (send4(t->px, t->py, t->pm, t->ps, false)) return 1;
         FA2_TRY(cudaMemcpyAsync(raw, t->reg, (size_t) t->nreg * sizeof(fa2_region),
                                 cudaMemcpyHostToDevice, s),
                 "the computation on the GPU failed", 1);

@@ -1,9 +1,11 @@
 """The all-pairs repulsion at the edges of its blocks, tiles and rows of
 sources. In double every node's terms are added in ascending order of the
-source, as the reference adds them: equal bits."""
+source, as the reference adds them: equal bits. In single the path's own bars,
+1e-4 norm-wise and 2e-3 with prevent_overlap, of the double forces."""
 import numpy as np
 import pytest
 
+from conftest import rel_err
 from forceatlas2_rc_gb300.layout import REPULSION_EXACT, Graph, Layout
 
 pytestmark = pytest.mark.gpu
@@ -28,3 +30,21 @@ def test_exact_double_bits(gpu, orc, n, adjust):
         got = L.forces(pos)
     want = orc.repulse_exact(n, pos, g.mass, size, adjust, 2.5)
     np.testing.assert_array_equal(got, np.asarray(want).reshape(got.shape))
+
+
+@pytest.mark.parametrize("adjust", [False, True])
+@pytest.mark.parametrize("n", [1, 2, 3, 15, 16, 31, 33, 255, 257, 512, 513, 1025, 4095, 4096,
+                               4097, 6145, 11999, 12000])
+def test_exact_single(gpu, n, adjust):
+    _, pos, _, double = _layout(n, "double", adjust, np.random.default_rng(n))
+    with double as L:
+        want = L.forces(pos)
+    _, _, _, single = _layout(n, "single", adjust, np.random.default_rng(n))
+    with single as L:
+        assert rel_err(L.forces(pos), want) <= (2e-3 if adjust else 1e-4)
+        L.iterate(2)  # the rows added up in the totals' launch
+        L.sync()
+        moved = L.positions()
+        L.set_positions(pos)
+        assert rel_err(L.forces(pos), want) <= (2e-3 if adjust else 1e-4)
+    assert np.isfinite(moved).all()
