@@ -49,21 +49,38 @@ enum {
 // predecessor still needs.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// `cluster` blocks to a thread-block cluster (0: none).
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_k(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block,
-                            size_t smem, cudaStream_t s, Args... args)
+inline cudaError_t launch_cluster(int cluster, bool pdl, void (*kernel)(KArgs...), dim3 grid,
+                                  dim3 block, size_t smem, cudaStream_t s, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = pdl ? attr : nullptr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (pdl) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 0) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = (unsigned) cluster;
+        attr[na].val.clusterDim.y = 1;
+        attr[na++].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = (unsigned) na;
     return cudaLaunchKernelEx(&cfg, kernel, ((KArgs) args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_k(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block,
+                            size_t smem, cudaStream_t s, Args... args)
+{
+    return launch_cluster(0, pdl, kernel, grid, block, smem, s, ((KArgs) args)...);
 }
 
 // Nanoseconds of the GPU's global timer (bounds of every device-side wait).

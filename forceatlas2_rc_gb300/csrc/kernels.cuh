@@ -110,6 +110,42 @@ __device__ __forceinline__ R rep_factor(R d2, R mm, R ss, R scaling)
     return d2 > R(0) ? fdiv(scaling * mm, d2) : R(0);
 }
 
+__device__ __forceinline__ uint32_t smem_addr(const void *p)
+{
+    return (uint32_t) __cvta_generic_to_shared(p);
+}
+
+// ---- mbarriers -------------------------------------------------------------
+
+__device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count)
+                 : "memory");
+}
+
+__device__ __forceinline__ bool mbar_try(uint64_t *bar, unsigned phase)
+{
+    unsigned ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                 " selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok)
+                 : "r"(smem_addr(bar)), "r"(phase)
+                 : "memory");
+    return ok != 0;
+}
+
+// Wait for a phase of `bar`, for at most `limit_ns` nanoseconds.
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned phase,
+                                          unsigned long long limit_ns)
+{
+    if (mbar_try(bar, phase)) return true;
+    const unsigned long long t0 = global_ns();
+    for (;;) {
+        if (mbar_try(bar, phase)) return true;
+        if (global_ns() - t0 > limit_ns) return false;
+    }
+}
+
 // ---- block reductions -----------------------------------------------------
 
 template <class T> __device__ __forceinline__ T warp_sum(T v)
@@ -293,6 +329,29 @@ __device__ __forceinline__ uint32_t morton_cell(float v, float m, double mn, dou
     return morton_cell((double) v, mn, scale);
 }
 
+// The quantisation of k_bbox, and the Morton code of a position by it.
+template <class R> struct MortonQuant {
+    double minx, miny, scale;
+    float4 qf = make_float4(0.f, 0.f, 0.f, 0.f);
+    __device__ __forceinline__ explicit MortonQuant(const double *quant)
+        : minx(quant[0]), miny(quant[1]), scale(quant[2])
+    {
+        if constexpr (sizeof(R) == 4) qf = *reinterpret_cast<const float4 *>(quant + 4);
+    }
+    __device__ __forceinline__ uint32_t key(typename RT<R>::R2 p) const
+    {
+        uint32_t cx, cy;
+        if constexpr (sizeof(R) == 4) {
+            cx = morton_cell(p.x, qf.z, minx, scale, qf.x, qf.y);
+            cy = morton_cell(p.y, qf.w, miny, scale, qf.x, qf.y);
+        } else {
+            cx = morton_cell(p.x, minx, scale);
+            cy = morton_cell(p.y, miny, scale);
+        }
+        return spread16(cx) | (spread16(cy) << 1);
+    }
+};
+
 // Morton codes and the identity order of the nodes (grid-stride). With
 // `aux` set, the same launch also makes the sort's digit histograms (its
 // histogram pass; the sort then starts with its scatter passes): launch few
@@ -306,9 +365,7 @@ k_morton(int n, const typename RT<R>::R2 *__restrict__ pos, const double *__rest
     __shared__ SortHistShared H;
     pdl_wait();
     if (aux) hist_begin(H, lookback, nlookback); // (uniform)
-    const double minx = quant[0], miny = quant[1], scale = quant[2];
-    float4 qf = make_float4(0.f, 0.f, 0.f, 0.f);
-    if constexpr (sizeof(R) == 4) qf = *reinterpret_cast<const float4 *>(quant + 4);
+    const MortonQuant<R> Q(quant);
     // U positions per thread loaded together, then coded
     constexpr int U = 4;
     const int stride = gridDim.x * blockDim.x;
@@ -321,21 +378,253 @@ k_morton(int n, const typename RT<R>::R2 *__restrict__ pos, const double *__rest
         for (int u = 0; u < U; u++) {
             const int i = i0 + u * stride;
             if (i >= n) break;
-            uint32_t cx, cy;
-            if constexpr (sizeof(R) == 4) {
-                cx = morton_cell(p[u].x, qf.z, minx, scale, qf.x, qf.y);
-                cy = morton_cell(p[u].y, qf.w, miny, scale, qf.x, qf.y);
-            } else {
-                cx = morton_cell(p[u].x, minx, scale);
-                cy = morton_cell(p[u].y, miny, scale);
-            }
-            const uint32_t k = spread16(cx) | (spread16(cy) << 1);
+            const uint32_t k = Q.key(p[u]);
             key[i] = k;
             idx[i] = (uint32_t) i;
             if (aux) hist_add(H, k, 4);
         }
     }
     if (aux) hist_end(H, 4, aux);
+}
+
+// ---- 2-3. codes and sort of a layout that fits one cluster's shared memory --
+// One cluster of thread blocks makes the codes of its nodes and sorts the
+// (code, node) pairs by four 8-bit digits, stable, without leaving shared
+// memory. Block b holds the pairs [b m, (b + 1) m) of the current order. A
+// pass: every warp ranks its contiguous pairs by digit (lane matching); the
+// blocks exchange their 256 digit counts through distributed shared memory;
+// each block orders its pairs by digit locally and writes them to their
+// places, in runs of equal digits, in the blocks that hold those places. The
+// last pass writes the sorted codes and nodes to global memory.
+//
+// Why: the tiled sort of such a layout is a launch for the codes and four of
+// 11-13 us each, all latency (3 to 25 tiles on 152 SMs). What bounds this: the
+// chain of a pass (rank, exchange of the counts, scatter), and above 50,000
+// nodes the scattered stores of 16 blocks. An iteration with the tiled sort
+// and with this, in us: 1,000 nodes 69 -> 62 (one-block sort), 3,001 94 -> 77,
+// 10,007 117 -> 90, 32,768 141 -> 121, 65,536 154 -> 143, 100,000 176 -> 174,
+// 131,072 187 -> 191. Counts and pairs are sent by asynchronous stores that
+// the receiver's mbarriers count (cluster barriers in their place: 2 us more
+// an iteration); as few threads as hold the pairs (512 and 1,024 threads at
+// 10,007 nodes: 94 and 97 us).
+constexpr int CS_MAX_BLOCKS = 16;
+constexpr int CS_MAX = 110000; // nodes up to which the cluster is the faster
+
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n"
+                 "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of a shared variable of block `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, unsigned rank)
+{
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// Asynchronous stores to shared memory of the cluster, counted in bytes by
+// the mbarrier of the block that is written to.
+__device__ __forceinline__ void cluster_store(uint32_t addr, uint32_t v, uint32_t bar)
+{
+    asm volatile(
+        "st.async.shared::cluster.mbarrier::complete_tx::bytes.u32 [%0], %1, [%2];" ::"r"(addr),
+        "r"(v), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void cluster_store2(uint32_t addr, uint2 v, uint32_t bar)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.u32 [%0], {%1, %2}, "
+                 "[%3];" ::"r"(addr),
+                 "r"(v.x), "r"(v.y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint64_t *bar, unsigned bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
+                 "r"(bytes)
+                 : "memory");
+}
+
+// T threads a block, at most ITEMS pairs a thread. Dynamic shared memory: two
+// arrays of m pairs.
+template <class R, int T, int ITEMS>
+__global__ void __launch_bounds__(T)
+k_codes_sort(int n, int m, const typename RT<R>::R2 *__restrict__ pos,
+             const double *__restrict__ quant, uint32_t *__restrict__ key,
+             uint32_t *__restrict__ order, int *__restrict__ status)
+{
+    constexpr int WARPS = T / 32, PARTS = T / 256; // threads a digit, eight warps each
+    extern __shared__ __align__(16) uint2 cs_pairs[];
+    // bytes of the counts, and of the pairs, that arrive in a pass: one phase
+    // of each a pass. A block sends a pass's counts when all its pairs of the
+    // pass before have come, and its pairs when all counts have: nobody
+    // writes what another still reads, nor into a phase not yet begun.
+    __shared__ uint64_t bar_counts, bar_pairs;
+    __shared__ uint32_t wh[WARPS][256];              // a warp's counts, then their prefix
+    __shared__ uint32_t table[2][CS_MAX_BLOCKS][256];   // the blocks' counts, by pass parity
+    __shared__ uint32_t lbase[256], gbase[256];
+    __shared__ uint2 wt[8];
+    const unsigned rank = blockIdx.x, blocks = gridDim.x; // one cluster
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int base = (int) rank * m, cnt = max(0, min(m, n - base));
+    unsigned below;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(below));
+    uint2 *A = cs_pairs, *B = cs_pairs + m;
+    // a warp's contiguous pairs: whole rounds of 32
+    const int rounds = (m + T - 1) / T; // <= ITEMS
+    const int first = w * rounds * 32;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar_counts, 1);
+        mbar_init(&bar_pairs, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    bool late = false;
+    pdl_wait();
+    {
+        const MortonQuant<R> Q(quant);
+        typename RT<R>::R2 p[ITEMS];
+#pragma unroll
+        for (int r = 0; r < ITEMS; r++) {
+            const int i = first + r * 32 + lane;
+            if (r < rounds && i < cnt) p[r] = pos[base + i];
+        }
+#pragma unroll
+        for (int r = 0; r < ITEMS; r++) {
+            const int i = first + r * 32 + lane;
+            if (r < rounds && i < cnt) A[i] = make_uint2(Q.key(p[r]), (uint32_t) (base + i));
+        }
+    }
+    // every block has started before another writes into it
+    cluster_barrier();
+    for (int pass = 0; pass < 4; pass++) {
+        const int shift = 8 * pass;
+        if (threadIdx.x == 0) {
+            mbar_expect(&bar_counts, blocks * 256u * (unsigned) sizeof(uint32_t));
+            if (pass < 3) mbar_expect(&bar_pairs, (unsigned) cnt * (unsigned) sizeof(uint2));
+        }
+#pragma unroll
+        for (int d = lane; d < 256; d += 32) wh[w][d] = 0;
+        __syncwarp();
+        uint2 item[ITEMS];
+        uint32_t rk[ITEMS];
+#pragma unroll
+        for (int r = 0; r < ITEMS; r++) {
+            if (r >= rounds) break; // (uniform)
+            const int i = first + r * 32 + lane;
+            const bool valid = i < cnt;
+            const unsigned act = __ballot_sync(0xffffffffu, valid);
+            item[r] = valid ? A[i] : make_uint2(0u, 0u);
+            const unsigned d = (item[r].x >> shift) & 255u;
+            uint32_t prior = 0, lt = 0, same = 0;
+            if (valid) {
+                const unsigned peers = match_digit8(act, d);
+                lt = __popc(peers & below);
+                same = __popc(peers);
+                prior = wh[w][d];
+            }
+            __syncwarp();
+            if (valid && lt == 0) wh[w][d] = prior + same;
+            __syncwarp();
+            rk[r] = prior + lt;
+        }
+        __syncthreads();
+        // per digit: the prefix over the warps and the
+        // block's count, sent to every block
+        {
+            const int d = threadIdx.x / PARTS, part = threadIdx.x % PARTS;
+            uint32_t c[8], run = 0;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                c[q] = wh[part * (8) + q][d];
+                run += c[q];
+            }
+            uint32_t incl = run;
+#pragma unroll
+            for (int o = 1; o < PARTS; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o, PARTS);
+                if (part >= o) incl += t;
+            }
+            uint32_t before = incl - run;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                wh[part * (8) + q][d] = before;
+                before += c[q];
+            }
+            const uint32_t all = __shfl_sync(0xffffffffu, incl, PARTS - 1, PARTS);
+            const uint32_t mine = smem_addr(&table[pass & 1][rank][d]);
+            const uint32_t bar = smem_addr(&bar_counts);
+            for (unsigned b = part; b < blocks; b += PARTS)
+                cluster_store(cluster_addr(mine, b), all, cluster_addr(bar, b));
+        }
+        late |= !mbar_wait(&bar_counts, pass & 1, 1000000000ull);
+        // global places: the digits in order, the blocks in order in a digit
+        uint32_t total = 0, prev = 0, own = 0, gincl = 0, lincl = 0;
+        if (threadIdx.x < 256) {
+#pragma unroll
+            for (unsigned b = 0; b < CS_MAX_BLOCKS; b++) {
+                const uint32_t c = b < blocks ? table[pass & 1][b][threadIdx.x] : 0u;
+                if (b < rank) prev += c;
+                if (b == rank) own = c;
+                total += c;
+            }
+            gincl = total;
+            lincl = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t g = __shfl_up_sync(0xffffffffu, gincl, o);
+                const uint32_t l = __shfl_up_sync(0xffffffffu, lincl, o);
+                if (lane >= o) {
+                    gincl += g;
+                    lincl += l;
+                }
+            }
+            if (lane == 31) wt[w] = make_uint2(gincl, lincl);
+        }
+        __syncthreads();
+        if (threadIdx.x < 256) {
+            uint32_t g = gincl - total + prev, l = lincl - own;
+#pragma unroll
+            for (int q = 0; q < 7; q++)
+                if (q < w) {
+                    g += wt[q].x;
+                    l += wt[q].y;
+                }
+            gbase[threadIdx.x] = g;
+            lbase[threadIdx.x] = l;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < ITEMS; r++) {
+            if (r >= rounds) break;
+            if (first + r * 32 + lane < cnt) {
+                const unsigned d = (item[r].x >> shift) & 255u;
+                const uint32_t at = lbase[d] + wh[w][d] + rk[r];
+                if (at < (uint32_t) cnt) A[at] = item[r]; // always, for consistent counts
+            }
+        }
+        __syncthreads();
+        const uint32_t there = smem_addr(B);
+        for (int i = threadIdx.x; i < cnt; i += T) {
+            const uint2 v = A[i];
+            const unsigned d = (v.x >> shift) & 255u;
+            const uint32_t g = gbase[d] + (uint32_t) i - lbase[d];
+            if (g >= (uint32_t) n) continue; // never, for consistent counts
+            if (pass == 3) {
+                key[g] = v.x;
+                order[g] = v.y;
+            } else {
+                const unsigned b = g / (unsigned) m;
+                cluster_store2(cluster_addr(there + 8u * (g - b * (unsigned) m), b), v,
+                               cluster_addr(smem_addr(&bar_pairs), b));
+            }
+        }
+        if (pass < 3) late |= !mbar_wait(&bar_pairs, pass & 1, 1000000000ull);
+        uint2 *t = A;
+        A = B;
+        B = t;
+    }
+    if (late) atomicOr(status + ST_ERROR, ERR_WAIT);
+    cluster_barrier(); // nobody leaves while another may still write to it
 }
 
 // ---- 4a. nodes in sorted order and the Karras tree (pipeline.cl:195-270) ----
@@ -992,11 +1281,6 @@ k_traverse_deferred(int n, R scaling, R theta2, double theta2d,
     if (k >= n) return;
     f[order[k]] = walk_deferred<R, ADJUST, COMP>(k, n, scaling, theta2, theta2d, psort, rec_c,
                                                  rec_t, agg, rope, status);
-}
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p)
-{
-    return (uint32_t) __cvta_generic_to_shared(p);
 }
 
 } // namespace fa2cu
@@ -2012,12 +2296,6 @@ k_pack_exact(int n, const double *__restrict__ x, const double *__restrict__ y,
 constexpr int EXACT_THREADS = 256;
 constexpr int EXACT_TILE = 256; // records (8 KB, double-buffered)
 
-__device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count)
-                 : "memory");
-}
-
 // Bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned)
 // from global to shared memory, completing on `bar`.
 __device__ __forceinline__ void tma_load_1d(void *dst, const void *src, unsigned bytes,
@@ -2031,29 +2309,6 @@ __device__ __forceinline__ void tma_load_1d(void *dst, const void *src, unsigned
             smem_addr(dst)),
         "l"(src), "r"(bytes), "r"(smem_addr(bar))
         : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(uint64_t *bar, unsigned phase)
-{
-    unsigned ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                 " selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok)
-                 : "r"(smem_addr(bar)), "r"(phase)
-                 : "memory");
-    return ok != 0;
-}
-
-// Wait for a phase of `bar`, for at most `limit_ns` nanoseconds.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned phase,
-                                          unsigned long long limit_ns)
-{
-    if (mbar_try(bar, phase)) return true;
-    const unsigned long long t0 = global_ns();
-    for (;;) {
-        if (mbar_try(bar, phase)) return true;
-        if (global_ns() - t0 > limit_ns) return false;
-    }
 }
 
 // Block (x, y) sums, for its EXACT_THREADS * IPT nodes, the sources [y seg,

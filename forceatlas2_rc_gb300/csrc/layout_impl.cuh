@@ -106,6 +106,59 @@ template <class R> struct Layout : LayoutBase {
     }
     int climb_mode = 1; // leaves per aggregate thread (negative: interleaved)
     bool block_sort = false; // few keys: the one-block sort
+    // blocks of the cluster that makes the codes and sorts them in one
+    // launch (0: codes and tiled sort), and its kernel's shape
+    int cluster = 0, cluster_shape = 0;
+    size_t cluster_smem() const { return 2 * sizeof(uint2) * (size_t) ceil_div(n, cluster); }
+    // Calls go(kernel, threads) for the shape that holds m pairs a block.
+    template <class F> static void with_cluster_kernel(int shape, F go)
+    {
+        switch (shape) {
+        case 0: return go(k_codes_sort<R, 256, 8>, 256);
+        case 1: return go(k_codes_sort<R, 512, 8>, 512);
+        default: return go(k_codes_sort<R, 512, 16>, 512);
+        }
+    }
+    static constexpr int cluster_pairs[3] = {2048, 4096, 8192};
+    // The shape for a cluster of c blocks: the first that holds the nodes.
+    bool pick_cluster(int c)
+    {
+        for (int shape = 0; shape < 3; shape++)
+            if (cluster_fits(n, c, shape)) {
+                cluster_shape = shape;
+                return true;
+            }
+        return false;
+    }
+    // Whether a cluster of c blocks of that shape runs on the current device
+    // with n nodes.
+    static bool cluster_fits(int n, int c, int shape)
+    {
+        if (c < 1 || c > CS_MAX_BLOCKS || ceil_div(n, c) > cluster_pairs[shape]) return false;
+        int fit = 0;
+        with_cluster_kernel(shape, [&](auto kernel, int threads) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned) c);
+            cfg.blockDim = dim3((unsigned) threads);
+            cfg.dynamicSmemBytes = 2 * sizeof(uint2) * (size_t) ceil_div(n, c);
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = (unsigned) c;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     2 * (int) sizeof(uint2) * cluster_pairs[shape]) !=
+                    cudaSuccess ||
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+                    cudaSuccess ||
+                cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                fit = 0;
+            }
+        });
+        return fit > 0;
+    }
 
     // Leaves per thread of the tree's climb, from the ratio x of leaves to
     // the threads the device holds at once (1536 per SM in float, 40
@@ -372,6 +425,10 @@ template <class R> struct Layout : LayoutBase {
             pdl = n < 500000;
             ss.pdl = pdl;
             block_sort = n <= SORT_BLOCK_MAX;
+            // (an iteration in us with 1 / 4 / 16 blocks: 100 nodes 40.5 / 42.2 /
+            // 44.3; 1,000 67.8 / 61.7 / 63.9; 3,001 - / 78.2 / 76.7)
+            const int c = n <= 256 ? 1 : n <= 2000 ? 4 : CS_MAX_BLOCKS;
+            if (n <= CS_MAX && pick_cluster(c)) cluster = c;
         }
         if (rep == FA2CU_REPULSION_EXACT) {
             int sms = 0;
@@ -474,6 +531,7 @@ template <class R> struct Layout : LayoutBase {
     // Morton codes, with the sort's digit histograms in the same launch
     void launch_build()
     {
+        if (cluster) return; // with the sort
         const int nb = std::min(ceil_div(n, 256), 152 * 4);
         if (block_sort) { // the one-block sort counts its own digits
             k_morton<R><<<nb, 256, 0, s>>>(n, pos, quant, key, order, nullptr, nullptr, 0);
@@ -487,7 +545,12 @@ template <class R> struct Layout : LayoutBase {
     }
     void launch_sort()
     {
-        if (block_sort)
+        if (cluster)
+            with_cluster_kernel(cluster_shape, [&](auto kernel, int threads) {
+                launch_cluster(cluster, pdl, kernel, dim3(cluster), dim3(threads), cluster_smem(),
+                               s, n, ceil_div(n, cluster), pos, quant, key, order, status);
+            });
+        else if (block_sort)
             sort_pairs_block(s, n, key, order, ss);
         else
             sort_pairs(s, n, key, order, ss, /*hist_ready=*/true);
@@ -941,8 +1004,19 @@ template <class R> struct Layout : LayoutBase {
             walk_split = (int) value;
             return recapture();
         }
+        if (!strcmp(name, "sort_cluster") && value >= 0 && value <= CS_MAX_BLOCKS &&
+            value == (int) value) {
+            const int c = (int) value;
+            if (c && !pick_cluster(c)) {
+                set_message("a cluster of %d blocks does not hold %d nodes", c, n);
+                return 1;
+            }
+            cluster = c;
+            return recapture();
+        }
         if (!strcmp(name, "sort_threads") && (value == 256 || value == 512 || value == 1024)) {
             ss.tile_threads = (int) value;
+            cluster = 0;
             return recapture();
         }
         if (!strcmp(name, "overlap") && (value == 0 || value == 1 || value == 2)) {
@@ -972,6 +1046,7 @@ template <class R> struct Layout : LayoutBase {
                 return 1;
             }
             block_sort = value == 1;
+            cluster = 0;
             return recapture();
         }
         if (!strcmp(name, "climb") &&

@@ -97,10 +97,14 @@ int fa2cu_layout_traversal_counts(fa2cu_layout *L, double counts[2]);
  *                  contiguous, -2 or -4 interleaved over the warp (default:
  *                  1 below one wave of threads, else 2 in float, 4 in
  *                  double);
- *   "sort_threads" 256, 512 or 1024 threads per sort tile (default: 512
- *                  below 600000 nodes, else 1024);
- *   "sort_block"   1: the one-block sort (at most 4096 nodes; default there),
- *                  0: the tiled sort;
+ *   "sort_cluster" blocks (1 to 16) of the cluster that makes the codes and
+ *                  sorts them in one launch (default: 1, 4 or 16 up to
+ *                  110,000 nodes); 0: separate launches;
+ *   "sort_threads" the tiled sort with 256, 512 or 1024 threads per tile
+ *                  (default above 110,000 nodes: 512 below 600000, else
+ *                  1024);
+ *   "sort_block"   1: the one-block sort (at most 4096 nodes), 0: the tiled
+ *                  sort;
  *   "keep_traction" 1: keep each node's traction of the last iteration for
  *                  fa2cu_layout_swing (n more reals on the device);
  *   "overlap"      single precision, Barnes-Hut: 1 gravity and attraction
