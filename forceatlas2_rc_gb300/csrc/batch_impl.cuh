@@ -330,7 +330,7 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
                 for (int q = 0; q < per; q++) {
                     const int k = tid * per + q;
                     if (k < n)
-                        climb<R, true>(k, n, psort, child, parent, range, rope, visits, agg,
+                        climb<R>(k, n, psort, child, parent, range, rope, visits, agg,
                                        rec_c, rec_t, wscale, status);
                 }
                 __syncthreads();

@@ -627,44 +627,10 @@ k_codes_sort(int n, int m, const typename RT<R>::R2 *__restrict__ pos,
     cluster_barrier(); // nobody leaves while another may still write to it
 }
 
-// ---- 4a. nodes in sorted order and the Karras tree (pipeline.cl:195-270) ----
-
-// The gather and the Karras tree in one launch: thread k writes sorted
-// node k's record and builds region k (both read only the sort's output).
-template <class R>
-__global__ void __launch_bounds__(256)
-k_gather_karras(int n, int adjust, const uint32_t *__restrict__ order,
-                const typename RT<R>::R2 *__restrict__ pos, const R *__restrict__ mass,
-                const R *__restrict__ size, typename RT<R>::R4 *__restrict__ psort,
-                const uint32_t *__restrict__ key, int2 *__restrict__ child,
-                int2 *__restrict__ range, int *__restrict__ parent, int *__restrict__ rope,
-                int *__restrict__ visits, int *__restrict__ status)
-{
-    pdl_wait();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    // the node's record is loaded first, so that its scattered loads are in
-    // flight during the tree search
-    const uint32_t i = order[k];
-    const bool ok = i < (uint32_t) n; // always, for a valid sort
-    typename RT<R>::R2 p = mk2<R>(R(0), R(0));
-    R m = R(0), sz = R(0);
-    if (ok) {
-        p = pos[i];
-        m = mass[i];
-        if (adjust) sz = size[i];
-    }
-    if (k < n - 1) karras_one<true>(k, n, key, child, range, parent, rope, visits);
-    if (!ok) atomicOr(status + ST_ERROR, ERR_BOUNDS);
-    psort[k] = mk4<R>(p.x, p.y, m, sz);
-}
-
-// ---- 4c. bottom-up centres of mass (pipeline.cl:272-323) -------------------
-// One thread per leaf climbs the tree; at each region, the first child to
-// arrive stops and the second computes the region from both children
-// (fixed order a then b: the sums do not depend on who arrives last). No
-// thread ever waits. The region's traversal record gets its skip link:
-// rope[last] is the right child of the region split just after `last`.
+// ---- 4. the tree's sums (pipeline.cl:272-323) -------------------------------
+// Each region's sums are made from its two children's, left then right, in a
+// fixed order whoever makes them: by the layouts' tree kernel (tree.cuh), and
+// by one climbing thread per leaf in the batched engine (climb, below).
 
 // ---- float-float arithmetic (error-free transformations) ------------------
 
@@ -748,6 +714,15 @@ __device__ __forceinline__ Agg<float> load_agg_cg(const Agg<float> *a)
     return v;
 }
 
+// Records that another block may have written in this launch.
+__device__ __forceinline__ float4 ldcg_r4(const float4 *p) { return __ldcg(p); }
+__device__ __forceinline__ double4_32a ldcg_r4(const double4_32a *p)
+{
+    const double2 *q = reinterpret_cast<const double2 *>(p);
+    const double2 a = __ldcg(q), b = __ldcg(q + 1);
+    return mk4<double>(a.x, a.y, b.x, b.y);
+}
+
 // The region from its two children, a then b (the order does not depend on
 // which child arrives last).
 __device__ __forceinline__ Agg<double> agg_combine(const Agg<double> &a, const Agg<double> &b)
@@ -809,39 +784,26 @@ __device__ __forceinline__ float4 agg_record(const Agg<float> &q, float wscale)
 
 // Arrival at region r: returns the number of children that arrived before
 // (0 or 1). acq_rel: the arriving thread's writes are visible before it
-// counts, and the second arrival sees the first's. CTA scope when one block
-// builds the whole tree (the batched engine), device scope otherwise.
-template <bool CTA> __device__ __forceinline__ int arrive(int *v)
+// counts, and the second arrival sees the first's (CTA scope: one block
+// builds the whole tree).
+__device__ __forceinline__ int arrive(int *v)
 {
     int prior;
-    if (CTA)
-        asm volatile("atom.add.acq_rel.cta.s32 %0, [%1], 1;" : "=r"(prior) : "l"(v) : "memory");
-    else
-        asm volatile("atom.add.acq_rel.gpu.s32 %0, [%1], 1;" : "=r"(prior) : "l"(v) : "memory");
+    asm volatile("atom.add.acq_rel.cta.s32 %0, [%1], 1;" : "=r"(prior) : "l"(v) : "memory");
     return prior;
 }
 
-// The climb of leaf k (sorted position) of an n-node tree: every region it
-// reaches second gets its sums (agg) and its traversal records.
-//
-// LOCAL: the block's threads climb from the leaves [s0, s1) (256 P of them),
-// so both arrivals at a region whose range lies in [s0, s1) come from this
-// block: they count on a shared-memory counter (shv[r - s0]; a Karras region
-// r always lies in its own range) at CTA scope, whose release costs a CTA
-// fence instead of the device-scope fence of a global counter. Only the
-// regions that span two blocks' leaves count on visits[] at device scope.
-// The data a second arrival reads (the sibling's sums) was written by the
-// thread that arrived first, before its release; which scope the counter has
-// changes neither the order of the sums nor the tree.
-template <class R, bool CTA, bool LOCAL = false>
+// The climb of leaf k (sorted position) of an n-node tree built by one block:
+// at each region, the first child to arrive stops and the second makes the
+// region's sums (agg) and traversal records. No thread ever waits. The
+// region's record gets its skip link: rope[last] is the right child of the
+// region split just after `last`.
+template <class R>
 __device__ __forceinline__ void climb(int k, int n, const typename RT<R>::R4 *psort,
-                                      const int2 *child,
-                                      const int *parent,
-                                      const int2 *range,
-                                      const int *rope, int *visits,
-                                      Agg<R> *agg, typename RT<R>::R4 *rec_c, int2 *rec_t,
-                                      R wscale, int *status, int *shv = nullptr, int s0 = 0,
-                                      int s1 = 0)
+                                      const int2 *child, const int *parent, const int2 *range,
+                                      const int *rope, int *visits, Agg<R> *agg,
+                                      typename RT<R>::R4 *rec_c, int2 *rec_t, R wscale,
+                                      int *status)
 {
     const int nl = n - 1;
     int r = parent[nl + k];
@@ -849,64 +811,13 @@ __device__ __forceinline__ void climb(int k, int n, const typename RT<R>::R4 *ps
     // the sibling's are loaded
     int prev = nl + k;
     Agg<R> mine = leaf_agg(psort[k]);
-    if (LOCAL) {
-        // the links of the region above (children, range, parent) are
-        // loaded as soon as the region is known, before the arrival there
-        // and while the current region's sums are made: one L2 round trip
-        // a level less on the chain of the climb
-        int2 c = make_int2(-1, -1), rg = make_int2(-1, -1);
-        int up = -1;
-        if ((unsigned) r < (unsigned) nl) {
-            c = child[r];
-            rg = range[r];
-            up = parent[r];
-        }
-        for (int depth = 0; r >= 0; depth++) {
-            if (r >= nl || depth > 160) {
-                atomicOr(status + ST_ERROR, ERR_BOUNDS);
-                return;
-            }
-            const bool here =
-                rg.x >= s0 && rg.y < s1 && (unsigned) (r - s0) < (unsigned) (s1 - s0);
-            if ((here ? arrive<true>(shv + (r - s0)) : arrive<false>(visits + r)) == 0) return;
-            int2 cn = make_int2(-1, -1), rgn = make_int2(-1, -1);
-            int upn = -1;
-            if ((unsigned) up < (unsigned) nl) {
-                cn = child[up];
-                rgn = range[up];
-                upn = parent[up];
-            }
-            if (c.x < 0 || c.y < 0 || c.x >= nl + n || c.y >= nl + n || rg.x < 0 ||
-                rg.y < 0 || rg.y >= n || (c.x != prev && c.y != prev)) {
-                atomicOr(status + ST_ERROR, ERR_BOUNDS);
-                return;
-            }
-            const int2 links =
-                make_int2(rg.y - rg.x >= 8 ? c.x : bucket_pack(rg.x, rg.y), rope[rg.y]);
-            const bool from_a = c.x == prev;
-            const int other = from_a ? c.y : c.x;
-            const Agg<R> o =
-                other >= nl ? leaf_agg(psort[other - nl]) : load_agg_cg(agg + other);
-            const Agg<R> q = from_a ? agg_combine(mine, o) : agg_combine(o, mine);
-            agg[r] = q;
-            rec_c[r] = agg_record(q, wscale);
-            rec_t[r] = links;
-            mine = q;
-            prev = r;
-            r = up;
-            c = cn;
-            rg = rgn;
-            up = upn;
-        }
-        return;
-    }
     // a Karras tree over 32-bit keys and n < 2^27 nodes is < 64 levels deep
     for (int depth = 0; r >= 0; depth++) {
         if (r >= nl || depth > 160) {
             atomicOr(status + ST_ERROR, ERR_BOUNDS);
             return;
         }
-        if (arrive<CTA>(visits + r) == 0) return;
+        if (arrive(visits + r) == 0) return;
         // the region's topology first (its links are known before its sums)
         const int2 c = child[r];
         const int2 rg = range[r];
@@ -933,61 +844,11 @@ __device__ __forceinline__ void climb(int k, int n, const typename RT<R>::R4 *ps
     }
 }
 
-template <class R>
-__global__ void __launch_bounds__(256)
-k_aggregate(int n, const typename RT<R>::R4 *__restrict__ psort,
-            const int2 *__restrict__ child, const int *__restrict__ parent,
-            const int2 *__restrict__ range, const int *__restrict__ rope,
-            int *__restrict__ visits, Agg<R> *__restrict__ agg,
-            typename RT<R>::R4 *__restrict__ rec_c, int2 *__restrict__ rec_t, R wscale,
-            int *__restrict__ status)
-{
-    __shared__ int shv[256];
-    shv[threadIdx.x] = 0;
-    pdl_wait();
-    __syncthreads();
-    const int s0 = blockIdx.x * 256, s1 = min(s0 + 256, n);
-    const int k = s0 + threadIdx.x;
-    if (k < n)
-        climb<R, false, true>(k, n, psort, child, parent, range, rope, visits, agg, rec_c,
-                              rec_t, wscale, status, shv, s0, s1);
-}
+} // namespace fa2cu
 
-// The climbs of P leaves per thread, one after the other: with n/P threads
-// the launch fits in fewer waves of blocks (1M leaves one per thread are 3.2
-// waves of 2048 threads on 152 SMs), and a climb no longer waits for a later
-// wave to finish the region above it. CONTIG: thread t takes leaves tP ..
-// tP+P-1; else lane l of warp w takes leaves (wP+q)32+l, q < P. Either way a
-// block takes the 256 P leaves from 256 P blockIdx.x on, whose inner regions
-// count their arrivals in shared memory. Which thread computes a region does
-// not change what it computes: the tree is the same. In float the launch
-// bound keeps 1536 threads per SM (40 registers: the early-loaded links of
-// the next level spill at 32), which the choice of P
-// (pick_climb) counts on.
-template <class R, int P, bool CONTIG>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 6 : 4)
-k_aggregate_multi(int n, const typename RT<R>::R4 *__restrict__ psort,
-                  const int2 *__restrict__ child, const int *__restrict__ parent,
-                  const int2 *__restrict__ range, const int *__restrict__ rope,
-                  int *__restrict__ visits, Agg<R> *__restrict__ agg,
-                  typename RT<R>::R4 *__restrict__ rec_c, int2 *__restrict__ rec_t, R wscale,
-                  int *__restrict__ status)
-{
-    __shared__ int shv[256 * P];
-#pragma unroll
-    for (int q = 0; q < P; q++) shv[q * 256 + threadIdx.x] = 0;
-    pdl_wait();
-    __syncthreads();
-    const int s0 = blockIdx.x * (256 * P), s1 = min(s0 + 256 * P, n);
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-#pragma unroll 1
-    for (int q = 0; q < P; q++) {
-        const int k = CONTIG ? t * P + q : ((t >> 5) * P + q) * 32 + (t & 31);
-        if (k < n)
-            climb<R, false, true>(k, n, psort, child, parent, range, rope, visits, agg, rec_c,
-                                  rec_t, wscale, status, shv, s0, s1);
-    }
-}
+#include "tree.cuh"
+
+namespace fa2cu {
 
 // ---- 5. Barnes-Hut traversal (pipeline.cl:329-383) -------------------------
 // One thread per node, in sorted order; the walk is stackless: from a region

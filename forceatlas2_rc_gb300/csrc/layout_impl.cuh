@@ -10,7 +10,7 @@
 //   key, order (+ ping-pong)  u32[n] x 4, look-back words u32[4 * 256 * n / 2048]
 //   psort               R4[n]   (x, y, m, r) in Morton order
 //   child, range        int2[n-1], parent int[2n-1], rope int[n],
-//   visits              int[n-1], agg Agg<R>[n-1] (double / float-float sums),
+//   meet                int[n-1], agg Agg<R>[n-1] (double / float-float sums),
 //                       rec_c R4[n-1], rec_t int2[n-1] (traversal records)
 //   bbox, quant         the bounding box and Morton quantisation, computed by
 //                       the displacement of the previous iteration
@@ -104,7 +104,6 @@ template <class R> struct Layout : LayoutBase {
         const double x = n / 32.0 / 5472.0; // of the device, with one warp each
         return x < 0.22 ? 4 : x < 0.45 ? 2 : 1;
     }
-    int climb_mode = 1; // leaves per aggregate thread (negative: interleaved)
     bool block_sort = false; // few keys: the one-block sort
     // blocks of the cluster that makes the codes and sorts them in one
     // launch (0: codes and tiled sort), and its kernel's shape
@@ -160,34 +159,18 @@ template <class R> struct Layout : LayoutBase {
         return fit > 0;
     }
 
-    // Leaves per thread of the tree's climb, from the ratio x of leaves to
-    // the threads the device holds at once (1536 per SM in float, 40
-    // registers). With block-local arrivals and the links of the next level
-    // loaded early (gather + Karras + climb in ms for 1 / 2 / 4 / 8 leaves
-    // per thread): BA 1e5 (x 0.43) 0.052 / 0.054 / 0.057 / 0.070; SBM 3e5
-    // (x 1.3) 0.071 / 0.066 / 0.066 / 0.078; 1e6 (x 4.3) 0.141 / 0.126 /
-    // 0.148 / 0.144; 3e6 0.346 / 0.276 / 0.287 / 0.405. Earlier build (2048
-    // threads per SM, device-scope arrivals only; climb alone, 1 / 2 / 4 / 8
-    // leaves per thread): 2e5 leaves (x 0.64) 0.069 / 0.074 / 0.084 / 0.123;
-    // 4e5 (x 1.3) 0.101 / 0.091 / 0.100 / 0.142; 6e5 (x 1.9) 0.128 / 0.107 /
-    // 0.117 / 0.155; 1e6 (x 3.2) 0.186 / 0.157 / 0.159 / 0.199; 2e6 (x 6.4)
-    // 0.326 / 0.263 / 0.289 / 0.387; 3e6 (x 9.6) 0.459 / 0.355 / 0.410 /
-    // 0.629. FP64 (fewer threads per SM): 4 leaves per thread was fastest or
-    // tied at 1e5 and 1e6 leaves (1e6: 0.554 / 0.382 / 0.334).
-    static int pick_climb(int n, int device)
+    // The tree's blocks search their edges in a window of 2 W leaves: a wide
+    // one shortens the climbs, which bound a small layout; a narrow one fills
+    // the blocks, of which a large one has many waves. An iteration in us with
+    // W 64 / 32: 10,007 nodes 69.8 / 71.6, 30,011 89.6 / 91.1, 100,000 156.4 /
+    // 153.4. The climbs in a launch of their own (32 and 16 then): 300,007 262
+    // in one / 264 apart, 10^6 666 / 641.
+    int tree_window = 64;
+    bool tree_apart = false;
+    void pick_tree()
     {
-        if (sizeof(R) == 8) return n >= 50000 ? 4 : 1;
-        int sms = 0, blocks = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_aggregate_multi<R, 2, true>,
-                                                          256, 0) !=
-                cudaSuccess ||
-            blocks < 1 || sms < 1) {
-            cudaGetLastError();
-            return 1;
-        }
-        const double x = (double) n / ((double) sms * blocks * 256.0);
-        return x < 1.0 ? 1 : 2;
+        tree_apart = n >= 400000;
+        tree_window = n < 60000 ? 64 : n < 400000 ? 32 : 16;
     }
     R scaling = 0, gravity = 0, theta2 = 0;
     R wscale = 0; // FP32 records: size^2 (1 + DECIDE_BAND) / theta^2 (region_far)
@@ -214,7 +197,9 @@ template <class R> struct Layout : LayoutBase {
     R2 *exact_part = nullptr; // exact_rows rows of partial sums (FP32, rows > 1)
     int exact_nrows = 1;
     int2 *child = nullptr, *range = nullptr;
-    int *parent = nullptr, *rope = nullptr, *visits = nullptr;
+    int *parent = nullptr, *rope = nullptr, *meet = nullptr;
+    int2 *piece = nullptr; // what climbs in the tree's second launch (tree.cuh)
+    int *pieces = nullptr;
     Agg<R> *agg = nullptr;
     R4 *rec_c = nullptr; // traversal records (common.cuh)
     int2 *rec_t = nullptr;
@@ -298,7 +283,10 @@ template <class R> struct Layout : LayoutBase {
             range = mem.get<int2>(nn - 1);
             parent = mem.get<int>(2 * nn - 1);
             rope = mem.get<int>(nn);
-            visits = mem.get<int>(nn - 1);
+            meet = mem.get<int>(nn - 1);
+            const size_t tree_blocks = (size_t) ceil_div(n, TREE_THREADS - 2 * 64);
+            piece = mem.get<int2>(tree_blocks * TREE_PIECES);
+            pieces = mem.get<int>(tree_blocks);
             agg = mem.get<Agg<R>>(nn - 1);
             rec_c = mem.get<R4>(nn - 1);
             rec_t = mem.get<int2>(nn - 1);
@@ -414,7 +402,8 @@ template <class R> struct Layout : LayoutBase {
         mem.s = s;
         if (rep == FA2CU_REPULSION_BH && sort_setup()) return 1;
         if (rep == FA2CU_REPULSION_BH) {
-            climb_mode = pick_climb(n, device);
+            pick_tree();
+            if (n > CS_MAX) attract_grid = 2;
             walk_split = pick_split(n);
             // sort tiles: fewer than ~75 tiles of 8192 keys leave most SMs
             // idle; measured on a GB300 (sort of one iteration, ms, tiles of
@@ -498,7 +487,12 @@ template <class R> struct Layout : LayoutBase {
         // whose reduction takes a ticket)
         FA2_TRY(cudaMemsetAsync(fold, 0, (size_t) n * sizeof(R2), s), "cudaMemset", 1);
         FA2_TRY(cudaMemsetAsync(status, 0, ST_COUNT * sizeof(int), s), "cudaMemset", 1);
-        if (repulsion == FA2CU_REPULSION_BH) sort_prepare(s, ss);
+        if (repulsion == FA2CU_REPULSION_BH) {
+            sort_prepare(s, ss);
+            // nobody has met at any split (each tree leaves them so)
+            FA2_TRY(cudaMemsetAsync(meet, 0xff, ((size_t) n - 1) * sizeof(int), s), "cudaMemset",
+                    1);
+        }
         if (set_positions(xy0)) return 1;
         SpeedState h{};
         h.speed = 1.0;
@@ -557,38 +551,25 @@ template <class R> struct Layout : LayoutBase {
     }
     void launch_tree()
     {
-        launch_k(pdl, k_gather_karras<R>, dim3(ceil_div(n, 256)), dim3(256), 0, s, n, adjust,
-                 order, pos, mass, size, psort, key, child, range, parent, rope, visits, status);
-        // every climb kernel waits for its predecessor before reading the tree
-        switch (climb_mode) {
-        case 2:
-            launch_k(pdl, k_aggregate_multi<R, 2, true>, dim3(ceil_div(n, 512)), dim3(256), 0, s,
-                     n, psort, child, parent, range, rope, visits, agg, rec_c, rec_t, wscale,
-                     status);
-            break;
-        case 4:
-            launch_k(pdl, k_aggregate_multi<R, 4, true>, dim3(ceil_div(n, 1024)), dim3(256), 0,
-                     s, n, psort, child, parent, range, rope, visits, agg, rec_c, rec_t, wscale,
-                     status);
-            break;
-        case 8:
-            launch_k(pdl, k_aggregate_multi<R, 8, true>, dim3(ceil_div(n, 2048)), dim3(256), 0,
-                     s, n, psort, child, parent, range, rope, visits, agg, rec_c, rec_t, wscale,
-                     status);
-            break;
-        case -2:
-            launch_k(pdl, k_aggregate_multi<R, 2, false>, dim3(ceil_div(n, 512)), dim3(256), 0,
-                     s, n, psort, child, parent, range, rope, visits, agg, rec_c, rec_t, wscale,
-                     status);
-            break;
-        case -4:
-            launch_k(pdl, k_aggregate_multi<R, 4, false>, dim3(ceil_div(n, 1024)), dim3(256), 0,
-                     s, n, psort, child, parent, range, rope, visits, agg, rec_c, rec_t, wscale,
-                     status);
-            break;
-        default:
-            launch_k(pdl, k_aggregate<R>, dim3(ceil_div(n, 256)), dim3(256), 0, s, n, psort,
-                     child, parent, range, rope, visits, agg, rec_c, rec_t, wscale, status);
+        // ranges and parents are made where something reads them
+        const bool full = walk == WALK_WARP;
+        full ? launch_tree_kernel<true>() : launch_tree_kernel<false>();
+    }
+    template <bool FULL> void launch_tree_kernel()
+    {
+        const TreeArrays<R> A{psort, rec_c, child, range, rec_t, parent, rope, meet, agg, piece,
+                              pieces};
+        const int blocks = ceil_div(n, TREE_THREADS - 2 * tree_window);
+        auto go = [&](auto kernel) {
+            launch_k(pdl, kernel, dim3(blocks), dim3(TREE_THREADS), 0, s, n, tree_window, adjust,
+                     order, pos, mass, size, key, A, wscale, status);
+        };
+        if (tree_apart) {
+            go(k_tree<R, FULL, true>);
+            launch_k(pdl, k_tree_top<R, FULL>, dim3(ceil_div(blocks, TREE_THREADS / 32)),
+                     dim3(TREE_THREADS), 0, s, n, blocks, key, A, wscale, status);
+        } else {
+            go(k_tree<R, FULL, false>);
         }
     }
     // (graphs with hubs: their walks add up with compensation)
@@ -736,12 +717,14 @@ template <class R> struct Layout : LayoutBase {
     }
     // FP32 Barnes-Hut: gravity and attraction into fatt, on stream s2
     // beside the tree build and the walk, added to the repulsion by the
-    // join (overlap 1: forked after the sort; 2: after the tree; 0: the
-    // attraction fused with the totals after the walk). Forked after the
-    // sort on one block per SM it measured 0.727 -> 0.711 ms an iteration at
-    // 10^6 SBM nodes, 0.229 -> 0.209 ms at 10^5 BA nodes; forked before the
-    // sort it delays the sort's tiles (0.77-0.85 ms, whatever the stream
-    // priorities), and more blocks per SM slow the walk.
+    // join (overlap 1: forked after the sort, or before the tiled sort's last
+    // pass; 2: after the tree; 0: the attraction fused with the totals after
+    // the walk). An iteration in us with 0 / 1 at 1 / 2 / 4 blocks an SM:
+    // 100,000 SBM nodes 162.5 / 157.6 / 158.9 / 160.7; 300,007 275.2 / 270.5 /
+    // 264.3 / 263.0; 10^6 670.7 / 642.9 / 649.6 / 655.0; 2,000,003 1233 / 1369 /
+    // 1206 / 1204. Forked at the iteration's start it delays the sort's tiles
+    // (10^6: 706 to 754); after the whole sort, the tree's blocks hold the SMs
+    // first (703).
     bool beside() const { return overlap && s2 && fatt && !serial_totals<R>(n); }
     // alone: nothing runs beside it (the force query, the phase times), one
     // thread per node; else attract_grid blocks per SM
@@ -770,9 +753,14 @@ template <class R> struct Layout : LayoutBase {
     {
         if (beside()) {
             launch_build();
+            // (with the tiled sort, before its last pass: the attraction's
+            // blocks are on the SMs before the tree's fill them)
+            const bool early = overlap == 1 && !cluster && !block_sort;
+            if (early) ss.before_last = ev_fork;
             launch_sort();
+            ss.before_last = nullptr;
             if (overlap == 2) launch_tree();
-            cudaEventRecord(ev_fork, s);
+            if (!early) cudaEventRecord(ev_fork, s);
             cudaStreamWaitEvent(s2, ev_fork, 0);
             launch_attraction_own(s2, false);
             cudaEventRecord(ev_join, s2);
@@ -957,7 +945,7 @@ template <class R> struct Layout : LayoutBase {
         if (set_positions(in)) return 1;
         launch_build();
         launch_sort();
-        launch_tree();
+        launch_tree_kernel<true>();
         std::vector<R4> hc((size_t) n - 1);
         std::vector<Agg<R>> ha(sizeof(R) == 4 ? (size_t) n - 1 : 0);
         const size_t nn = (size_t) n;
@@ -1052,7 +1040,7 @@ template <class R> struct Layout : LayoutBase {
         if (!strcmp(name, "climb") &&
             (value == 1 || value == 2 || value == 4 || value == 8 || value == -2 ||
              value == -4)) {
-            climb_mode = (int) value;
+            tree_apart = value != 1;
             return recapture();
         }
         if (!strcmp(name, "walk") &&

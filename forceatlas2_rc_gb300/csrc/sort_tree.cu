@@ -291,6 +291,7 @@ void sort_pairs_passes(cudaStream_t s, int n, uint32_t *key, uint32_t *val,
     }
     uint32_t *ka = key, *va = val, *kb = w.key_b, *vb = w.val_b;
     for (int pass = 0; pass < passes; pass++) {
+        if (pass == passes - 1 && w.before_last) cudaEventRecord(w.before_last, s);
         if (w.tile_threads == 1024)
             onesweep_pass<1024>(s, n, pass, ka, va, kb, vb, w);
         else if (w.tile_threads == 512)

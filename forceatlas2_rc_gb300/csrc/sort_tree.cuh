@@ -33,6 +33,7 @@ struct SortScratch {
     int *err = nullptr;
     int tile_threads = 1024; // threads of a scatter block (tile = 8 keys each)
     bool pdl = false;        // scatter passes launched as programmatic dependents
+    cudaEvent_t before_last = nullptr; // recorded before the last pass
 };
 size_t sort_scratch_counts(int n); // entries of `counts`
 

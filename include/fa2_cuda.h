@@ -93,10 +93,9 @@ int fa2cu_layout_traversal_counts(fa2cu_layout *L, double counts[2]);
  *   "walk_split"   single precision: warps that share the walk of 32 nodes,
  *                  1, 2 or 4 (default: 4 below 38,000 nodes, 2 below
  *                  79,000, else 1; forces equal to ~1e-7);
- *   "climb"        leaves per thread of the bottom-up sums: 1, 2, 4 or 8
- *                  contiguous, -2 or -4 interleaved over the warp (default:
- *                  1 below one wave of threads, else 2 in float, 4 in
- *                  double);
+ *   "climb"        1: the tree in one launch; 2, 4, 8, -2 or -4: the regions
+ *                  that span its blocks in a second one (default from
+ *                  400,000 nodes; the same tree);
  *   "sort_cluster" blocks (1 to 16) of the cluster that makes the codes and
  *                  sorts them in one launch (default: 1, 4 or 16 up to
  *                  110,000 nodes); 0: separate launches;
@@ -109,12 +108,14 @@ int fa2cu_layout_traversal_counts(fa2cu_layout *L, double counts[2]);
  *                  fa2cu_layout_swing (n more reals on the device);
  *   "overlap"      single precision, Barnes-Hut: 1 gravity and attraction
  *                  computed on a second stream beside the tree build and
- *                  the walk (forked after the sort; default), into a buffer
- *                  of their own that is then added to the repulsion; 2 the
- *                  same forked after the tree build; 0 the attraction after
+ *                  the walk (forked after the sort, or before the last pass
+ *                  of the tiled sort; default), into a buffer of their own
+ *                  that is then added to the repulsion; 2 the same forked
+ *                  after the tree build; 0 the attraction after
  *                  the walk, added to the repulsion node by node (forces
  *                  equal to ~1e-7);
- *   "attract_grid" blocks per SM of that attraction, 1 (default) to 8;
+ *   "attract_grid" blocks per SM of that attraction, 1 to 8 (default 1, 2
+ *                  above 110,000 nodes);
  *   "join_blocks"  blocks of 256 threads of the join that adds it to the
  *                  repulsion and sums the swing totals (default 608: few
  *                  block partials for its last block);
