@@ -97,23 +97,22 @@ template <int W> __device__ double block_sum(double v, double *scratch)
 
 // ---- the persistent kernel -----------------------------------------------------
 
-// FP32: three blocks of 512 (six of 256) threads per SM, 40 registers a
-// thread (~120 bytes of spills, in the sort and tree phases): 48 warps
-// resident for the walk, which is bound by instruction issue. Against two
-// blocks of 512 at 63 registers: 7.30 -> 6.49 ms a batch iteration of 4096
-// graphs; four blocks (32 registers, ~400 bytes of spills) 6.60-6.70 ms.
-// FP64 needs more registers: one block of 512 (two of 256).
+// FP32: two blocks of 512 (four of 256) threads per SM, 64 registers a thread,
+// which the group walk wants (three blocks at 40 registers: 3.01 against 2.85
+// ms an iteration of 1,024 graphs of 50 to 20,000 nodes). FP64 needs more registers: one block of 512 (two
+// of 256).
 template <class R, int T>
-__global__ void __launch_bounds__(T, (sizeof(R) == 8 ? 512 : 1536) / T)
+__global__ void __launch_bounds__(T, (sizeof(R) == 8 ? 512 : 1024) / T)
 k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterations,
         BatchArrays<R> A, int npt, int *status)
 {
     typedef typename RT<R>::R2 R2;
     typedef typename RT<R>::R4 R4;
     constexpr int W = T / 32;
-    // the sort's digit counts; the exact sum's record tile (T records of at
-    // most 32 bytes) in the same space
-    __shared__ __align__(16) uint32_t cnt[W][256];
+    // the sort's digit counts; in the same space the exact sum's record tile
+    // (T records of at most 32 bytes), and the group walk's arrays
+    extern __shared__ __align__(16) unsigned char batch_smem[];
+    uint32_t(*cnt)[256] = reinterpret_cast<uint32_t(*)[256]>(batch_smem);
     __shared__ uint32_t dbase[256];
     __shared__ double red[W], red2[W];
     __shared__ R mins[4][W];
@@ -335,33 +334,50 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
                 }
                 __syncthreads();
                 phase(BP_SUMS);
-                // FP32: the walk with its node pairs deferred (the single
-                // layout's), compensated for hubs; FP64: the per-thread walk
-                // in the reference's order
-                for (int k = tid; k < n; k += T) {
-                    R2 fk;
-                    if constexpr (sizeof(R) == 4) {
-                        if (hubs)
-                            fk = adjust ? walk_deferred<R, true, true>(k, n, scaling, theta2,
-                                                                       theta2d, psort, rec_c,
-                                                                       rec_t, agg, rope, status)
-                                        : walk_deferred<R, false, true>(k, n, scaling, theta2,
-                                                                        theta2d, psort, rec_c,
-                                                                        rec_t, agg, rope, status);
-                        else
-                            fk = adjust ? walk_deferred<R, true>(k, n, scaling, theta2, theta2d,
-                                                                 psort, rec_c, rec_t, agg, rope,
-                                                                 status)
-                                        : walk_deferred<R, false>(k, n, scaling, theta2, theta2d,
-                                                                  psort, rec_c, rec_t, agg, rope,
-                                                                  status);
-                    } else {
-                        fk = adjust ? walk<R, true>(k, n, scaling, theta2, theta2d, psort, rec_c,
-                                                    rec_t, agg, rope, status)
-                                    : walk<R, false>(k, n, scaling, theta2, theta2d, psort, rec_c,
-                                                     rec_t, agg, rope, status);
-                    }
-                    f[idx[k]] = fk;
+                // FP32: the group walk (the single layout's), compensated for
+                // hubs, every warp from the root: a block's shared top is a
+                // barrier that few blocks an SM do not hide (3.02 against 2.85
+                // ms; with one walk a thread 3.70). FP64: the per-thread walk
+                // in the reference's order.
+                if constexpr (sizeof(R) == 4) {
+                    GroupTopShared &top = *reinterpret_cast<GroupTopShared *>(batch_smem);
+                    GroupWalkShared *gw = reinterpret_cast<GroupWalkShared *>(&top + 1);
+                    auto go = [&](auto walk_block) {
+                        for (int k0 = 0; k0 < n; k0 += T) {
+                            const R2 fk = walk_block(k0);
+                            if (k0 + tid < n) f[idx[k0 + tid]] = fk;
+                        }
+                    };
+                    if (adjust && hubs)
+                        go([&](int k0) {
+                            return group_walk_block<true, true>(top, gw, k0, 1, false, n, scaling, theta2d,
+                                                                psort, rec_c, rec_t, child, agg,
+                                                                status);
+                        });
+                    else if (adjust)
+                        go([&](int k0) {
+                            return group_walk_block<true, false>(top, gw, k0, 1, false, n, scaling,
+                                                                 theta2d, psort, rec_c, rec_t,
+                                                                 child, agg, status);
+                        });
+                    else if (hubs)
+                        go([&](int k0) {
+                            return group_walk_block<false, true>(top, gw, k0, 1, false, n, scaling,
+                                                                 theta2d, psort, rec_c, rec_t,
+                                                                 child, agg, status);
+                        });
+                    else
+                        go([&](int k0) {
+                            return group_walk_block<false, false>(top, gw, k0, 1, false, n, scaling,
+                                                                  theta2d, psort, rec_c, rec_t,
+                                                                  child, agg, status);
+                        });
+                } else {
+                    for (int k = tid; k < n; k += T)
+                        f[idx[k]] = adjust ? walk<R, true>(k, n, scaling, theta2, theta2d, psort,
+                                                           rec_c, rec_t, agg, rope, status)
+                                           : walk<R, false>(k, n, scaling, theta2, theta2d, psort,
+                                                            rec_c, rec_t, agg, rope, status);
                 }
             }
             __syncthreads();
@@ -455,6 +471,15 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
             G->efficiency = eff;
         }
     }
+}
+
+// Dynamic shared memory of k_batch.
+template <class R, int T> constexpr size_t batch_smem_bytes()
+{
+    const size_t sort = (size_t) (T / 32) * 256 * sizeof(uint32_t);
+    const size_t walk =
+        sizeof(R) == 4 ? sizeof(GroupTopShared) + (T / 32) * sizeof(GroupWalkShared) : 0;
+    return sort > walk ? sort : walk;
 }
 
 // ---- host side -------------------------------------------------------------------
@@ -622,10 +647,16 @@ template <class R> struct Batch : BatchBase {
         }
         int sms = 0, per_sm = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        if (threads == 256)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<R, 256>, 256, 0);
-        else
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<R, 512>, 512, 0);
+        auto setup = [&](auto kernel, int th, size_t smem) {
+            FA2_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int) smem),
+                    "cudaFuncSetAttribute", 1);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, th, smem);
+            return 0;
+        };
+        if (threads == 256 ? setup(k_batch<R, 256>, 256, batch_smem_bytes<R, 256>())
+                           : setup(k_batch<R, 512>, 512, batch_smem_bytes<R, 512>()))
+            return 1;
         blocks = std::max(1, std::min(G, sms * std::max(per_sm, 1)));
         return 0;
     }
@@ -638,15 +669,20 @@ template <class R> struct Batch : BatchBase {
         return v;
     }
 
+    void launch_kernel(int iterations, const BatchArrays<R> &arrays)
+    {
+        if (threads == 256)
+            k_batch<R, 256><<<blocks, 256, batch_smem_bytes<R, 256>(), s>>>(
+                G, graphs, queue, next, iterations, arrays, npt, status);
+        else
+            k_batch<R, 512><<<blocks, 512, batch_smem_bytes<R, 512>(), s>>>(
+                G, graphs, queue, next, iterations, arrays, npt, status);
+    }
+
     void launch(int iterations)
     {
         cudaMemsetAsync(next, 0, sizeof(int), s);
-        if (threads == 256)
-            k_batch<R, 256><<<blocks, 256, 0, s>>>(G, graphs, queue, next, iterations, A, npt,
-                                                   status);
-        else
-            k_batch<R, 512><<<blocks, 512, 0, s>>>(G, graphs, queue, next, iterations, A, npt,
-                                                   status);
+        launch_kernel(iterations, A);
     }
 
     // The work-counter reset and the persistent launch, captured once per
@@ -697,14 +733,7 @@ template <class R> struct Batch : BatchBase {
         BatchArrays<R> P = A;
         P.prof = prof;
         if (!rc) rc = cudaMemsetAsync(next, 0, sizeof(int), s) != cudaSuccess;
-        if (!rc) {
-            if (threads == 256)
-                k_batch<R, 256><<<blocks, 256, 0, s>>>(G, graphs, queue, next, iterations, P,
-                                                       npt, status);
-            else
-                k_batch<R, 512><<<blocks, 512, 0, s>>>(G, graphs, queue, next, iterations, P,
-                                                       npt, status);
-        }
+        if (!rc) launch_kernel(iterations, P);
         std::vector<unsigned long long> h((size_t) blocks * 8);
         if (!rc)
             rc = cudaMemcpyAsync(h.data(), prof, h.size() * sizeof(unsigned long long),

@@ -150,8 +150,8 @@ template <> struct GroupAcc<true> {
     float ax = 0.0f, ay = 0.0f, cx = 0.0f, cy = 0.0f;
     __device__ __forceinline__ void add(float xd, float yd, float g)
     {
-        acc_add(ax, cx, xd * g, true);
-        acc_add(ay, cy, yd * g, true);
+        acc_add(ax, cx, xd * g);
+        acc_add(ay, cy, yd * g);
     }
     __device__ __forceinline__ void add2(f2 xd, f2 yd, f2 g)
     {
@@ -288,7 +288,7 @@ __device__ __forceinline__ void group_pairs(GroupWalkShared &S, int nb, int n, c
             unsigned lanes = 0;
             if (i < total) {
                 const int2 f = S.flat[i];
-                p = ldg_r4(psort + f.x);
+                p = psort[f.x];
                 lanes = (unsigned) f.y;
             }
             NodePair &t = S.node[i >> 1];
@@ -376,9 +376,9 @@ __device__ __forceinline__ void group_top(GroupTopShared &T, GroupWalkShared &S,
         float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         int2 ch = make_int2(0, 0);
         if ((unsigned) r < (unsigned) nl) {
-            c = ldg_r4(rec_c + r);
-            const int left = __ldg(&rec_t[r].x);
-            ch = __ldg(child + r);
+            c = rec_c[r];
+            const int left = rec_t[r].x;
+            ch = child[r];
             verdict = box_test(box, c, c.w * DECIDE_LO);
             if (verdict < 0 && left < 0) verdict = 0; // a bucket: left to the warps
         }
@@ -471,9 +471,9 @@ __device__ __forceinline__ void group_walk(const GroupTopShared &T, GroupWalkSha
         int verdict = 2; // 2: nothing; else box_test, and 0 for far from some lanes only
         float floor = 0.0f;
         if (lanes && (unsigned) e.x < (unsigned) nl) {
-            c = ldg_r4(rec_c + e.x);
-            t.x = __ldg(&rec_t[e.x].x);
-            ch = __ldg(child + e.x);
+            c = rec_c[e.x];
+            t.x = rec_t[e.x].x;
+            ch = child[e.x];
             floor = c.w * DECIDE_LO;
             verdict = box_test(box, c, floor);
             if (verdict > 0 && lanes != all) verdict = 0;
@@ -578,14 +578,18 @@ __device__ __forceinline__ void group_walk(const GroupTopShared &T, GroupWalkSha
     group_pairs<ADJUST, COMP>(S, nb, n, own, me, psort, acc, status);
 }
 
+// (The tree is read by plain loads: the batched engine makes it in the same
+// launch.)
 // The walk of one block's nodes, 32 to each `split` of its warps, which share
 // the regions left by group_top: the force of node base0 + 32 (w / split) +
 // lane in the lanes of warp w (valid below n and where w % split is 0).
-// Every thread of the block calls it. HUBS: the graph has nodes of HUB_MASS
+// Without shared_top (split 1) every warp starts at the root, and no barrier is
+// met. Every thread of the block calls it. HUBS: the graph has nodes of HUB_MASS
 // or more; a warp that holds one adds up with compensation.
 template <bool ADJUST, bool HUBS>
 __device__ __forceinline__ float2
-group_walk_block(GroupTopShared &T, GroupWalkShared *Sw, int base0, int split, int n,
+group_walk_block(GroupTopShared &T, GroupWalkShared *Sw, int base0, int split, bool shared_top,
+                 int n,
                  float scaling, double theta2d, const float4 *psort, const float4 *rec_c,
                  const int2 *rec_t, const int2 *child, const Agg<float> *agg, int *status)
 {
@@ -595,12 +599,20 @@ group_walk_block(GroupTopShared &T, GroupWalkShared *Sw, int base0, int split, i
     const int k = min(base + lane, n - 1);
     const float4 own = psort[k];
     const float4 box = warp_box(make_float4(own.x, own.y, own.x, own.y));
-    if (lane == 0) T.box[w] = box;
-    __syncthreads();
     GroupWalkShared &S = Sw[w];
-    if (w == 0) // (a warp past the end holds node n - 1's box)
-        group_top(T, S, n, warp_box(T.box[min(lane, warps - 1)]), rec_c, rec_t, child);
-    __syncthreads();
+    if (shared_top) {
+        if (lane == 0) T.box[w] = box;
+        __syncthreads();
+        if (w == 0) // (a warp past the end holds node n - 1's box)
+            group_top(T, S, n, warp_box(T.box[min(lane, warps - 1)]), rec_c, rec_t, child);
+        __syncthreads();
+    } else {
+        if (lane == 0) {
+            T.box[w] = box;
+            T.nroot = -1; // (the same value from every warp)
+        }
+        __syncwarp();
+    }
     float2 v = make_float2(0.0f, 0.0f);
     if (base < n) {
         if (HUBS && __any_sync(0xffffffffu, own.z >= HUB_MASS)) {

@@ -994,46 +994,37 @@ k_traverse(int n, R scaling, R theta2, double theta2d,
                                   rope, status);
 }
 
-// The walk with its node pairs deferred (the batched FP32 layouts). In the
-// walk above, a
-// warp whose lanes are partly summing node pairs and partly visiting
-// regions issues both kinds of step in nearly every iteration. Here the walk
-// visits regions only: a small region that is too close (and a single node
-// reached as a leaf) is queued as its packed sorted range, and the queued
-// node pairs are summed after the walk -- before, if the queue fills up.
-// The regions and the pairs are those of walk(); the force is summed in
-// another order: the far regions in walk order, then the pairs in walk order.
+// The walk with its node pairs deferred. In the walk above, a warp whose lanes
+// are partly summing node pairs and partly visiting regions issues both kinds
+// of step in nearly every iteration. Here the walk visits regions only: a
+// small region that is too close (and a single node reached as a leaf) is
+// queued as its packed sorted range, and the queued node pairs are summed
+// after the walk -- before, if the queue fills up. The regions and the pairs
+// are those of walk(); the force is summed in another order: the far regions
+// in walk order, then the pairs in walk order. (In float the group walk takes
+// its place.)
 constexpr int DEFER_QUEUE = 16;
 
 // A node of mass 1 + HEAVY_DEGREE or more (a hub) near equilibrium feels a
 // repulsion that nearly cancels an attraction ~100 times larger than the
 // net force: summed in plain float, the running sum's roundings reach
-// ~1e-4 of the largest net force. The walk adds its terms with Kahan
-// compensation for such nodes (in graphs that have any; COMP).
+// ~1e-4 of the largest net force. The group walk adds its terms with Kahan
+// compensation for such nodes (in graphs that have any).
 constexpr float HUB_MASS = 1.0f + 128; // 1 + HEAVY_DEGREE (below)
 
-// s += v, compensated when `comp` (c carries the lost low part, negated).
-__device__ __forceinline__ void acc_add(float &s, float &c, float v, bool comp)
+// s += v, compensated (c carries the lost low part, negated).
+__device__ __forceinline__ void acc_add(float &s, float &c, float v)
 {
-    if (comp) {
-        const float y = __fsub_rn(v, c);
-        const float t = __fadd_rn(s, y);
-        c = __fsub_rn(__fsub_rn(t, s), y);
-        s = t;
-    } else {
-        s += v;
-    }
+    const float y = __fsub_rn(v, c);
+    const float t = __fadd_rn(s, y);
+    c = __fsub_rn(__fsub_rn(t, s), y);
+    s = t;
 }
-__device__ __forceinline__ void acc_add(double &s, double &, double v, bool) { s += v; }
-
-// Read-only loads of the walk's inputs (non-coherent path in float).
-__device__ __forceinline__ float4 ldg_r4(const float4 *p) { return __ldg(p); }
-__device__ __forceinline__ double4_32a ldg_r4(const double4_32a *p) { return *p; }
 
 template <class R, bool ADJUST>
 __device__ __forceinline__ void sum_pairs(int k, const int *q, int nq, R xi, R yi, R mi, R si,
                                           R scaling, const typename RT<R>::R4 *psort, R &ax,
-                                          R &ay, R &cx, R &cy, bool comp)
+                                          R &ay)
 {
     // one loop over all the queued pairs (bucket after bucket, each in
     // sorted order): the lanes of a warp run as many iterations as the
@@ -1042,11 +1033,11 @@ __device__ __forceinline__ void sum_pairs(int k, const int *q, int nq, R xi, R y
     int b = 0, j = bucket_first(q[0]), last = bucket_last(q[0]);
     for (;;) {
         if (j != k) {
-            const typename RT<R>::R4 p = ldg_r4(psort + j);
+            const typename RT<R>::R4 p = psort[j];
             const R xd = xi - p.x, yd = yi - p.y;
             const R g = rep_factor<R, ADJUST>(sq_dist(xd, yd), mi * p.z, si + p.w, scaling);
-            acc_add(ax, cx, xd * g, comp);
-            acc_add(ay, cy, yd * g, comp);
+            ax += xd * g;
+            ay += yd * g;
         }
         if (++j > last) {
             if (++b >= nq) break;
@@ -1056,7 +1047,7 @@ __device__ __forceinline__ void sum_pairs(int k, const int *q, int nq, R xi, R y
     }
 }
 
-template <class R, bool ADJUST, bool COMP = false>
+template <class R, bool ADJUST>
 __device__ __forceinline__ typename RT<R>::R2
 walk_deferred(int k, int n, R scaling, R theta2, double theta2d,
               const typename RT<R>::R4 *psort, const typename RT<R>::R4 *rec_c,
@@ -1067,8 +1058,7 @@ walk_deferred(int k, int n, R scaling, R theta2, double theta2d,
     const R xi = me.x, yi = me.y, mi = me.z, si = me.w;
     // a far region's pull is (scaling m_i) m / d^2
     const R smi = scaling * mi;
-    R ax = R(0), ay = R(0), cx = R(0), cy = R(0);
-    const bool comp = COMP && sizeof(R) == 4 && mi >= R(HUB_MASS);
+    R ax = R(0), ay = R(0);
     const int nl = n - 1;
     const unsigned nend = (unsigned) (nl + n);
     int q[DEFER_QUEUE];
@@ -1089,18 +1079,18 @@ walk_deferred(int k, int n, R scaling, R theta2, double theta2d,
             }
             const int j = cur - nl; // a single node
             bucket = bucket_pack(j, j);
-            cur = __ldg(rope + j);
+            cur = rope[j];
         } else {
-            const R4 c = ldg_r4(rec_c + cur);
-            const int2 t = __ldg(rec_t + cur);
+            const R4 c = rec_c[cur];
+            const int2 t = rec_t[cur];
             const R xd = xi - c.x, yd = yi - c.y;
             const R d2 = sq_dist(xd, yd);
             const bool far =
                 region_far(d2, c.w, theta2, agg + cur, (float) xi, (float) yi, theta2d);
             if (far) {
                 const R g = fdiv(smi * c.z, d2);
-                acc_add(ax, cx, xd * g, comp);
-                acc_add(ay, cy, yd * g, comp);
+                ax += xd * g;
+                ay += yd * g;
                 cur = t.y;
                 continue;
             }
@@ -1116,20 +1106,16 @@ walk_deferred(int k, int n, R scaling, R theta2, double theta2d,
             cur = t.y;
         }
         if (nq == DEFER_QUEUE) {
-            sum_pairs<R, ADJUST>(k, q, nq, xi, yi, mi, si, scaling, psort, ax, ay, cx, cy, comp);
+            sum_pairs<R, ADJUST>(k, q, nq, xi, yi, mi, si, scaling, psort, ax, ay);
             nq = 0;
         }
         q[nq++] = bucket;
     }
-    sum_pairs<R, ADJUST>(k, q, nq, xi, yi, mi, si, scaling, psort, ax, ay, cx, cy, comp);
-    if (comp) {
-        ax -= cx;
-        ay -= cy;
-    }
+    sum_pairs<R, ADJUST>(k, q, nq, xi, yi, mi, si, scaling, psort, ax, ay);
     return mk2<R>(ax, ay);
 }
 
-template <class R, bool ADJUST, int MINB, bool COMP = false>
+template <class R, bool ADJUST, int MINB>
 __global__ void __launch_bounds__(256, MINB)
 k_traverse_deferred(int n, R scaling, R theta2, double theta2d,
                     const typename RT<R>::R4 *__restrict__ psort,
@@ -1140,8 +1126,8 @@ k_traverse_deferred(int n, R scaling, R theta2, double theta2d,
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    f[order[k]] = walk_deferred<R, ADJUST, COMP>(k, n, scaling, theta2, theta2d, psort, rec_c,
-                                                 rec_t, agg, rope, status);
+    f[order[k]] = walk_deferred<R, ADJUST>(k, n, scaling, theta2, theta2d, psort, rec_c, rec_t,
+                                           agg, rope, status);
 }
 
 } // namespace fa2cu
@@ -1165,7 +1151,7 @@ k_traverse_group(int n, int split, float scaling, double theta2d, const float4 *
     __shared__ GroupWalkShared S[GW_WARPS];
     pdl_wait();
     const int base0 = blockIdx.x * (32 * GW_WARPS / split);
-    const float2 v = group_walk_block<ADJUST, HUBS>(T, S, base0, split, n, scaling, theta2d, psort,
+    const float2 v = group_walk_block<ADJUST, HUBS>(T, S, base0, split, true, n, scaling, theta2d, psort,
                                                     rec_c, rec_t, child, agg, status);
     const int w = threadIdx.x >> 5, k = base0 + 32 * (w / split) + (int) (threadIdx.x & 31);
     if (w % split == 0 && k < n) f[order[k]] = v;
