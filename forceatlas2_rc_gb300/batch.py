@@ -18,7 +18,7 @@ import numpy as np
 from . import _lib
 from ._abi import FullParams, dptr
 from ._lib import P_D
-from .layout import Graph, _cols, _params
+from .layout import Graph, _cols, _params, _rows
 
 
 def tune(device: int = 0, precision: str = "single") -> dict:
@@ -109,17 +109,17 @@ class Batch:
 
     def positions(self, g: int) -> np.ndarray:
         n = self.sizes[g]
-        xy = np.zeros(2 * n)
+        xy = np.empty(2 * n)
         self._check(self.lib.fa2cu_batch_positions(self.h, int(g), dptr(xy)))
-        return xy.reshape(2, n).T.copy()
+        return _rows(xy, n)
 
     def forces(self, g: int) -> np.ndarray:
         """Graph g's forces of the last iteration, at the positions before
         its displacement, as an (n, 2) array (after ``sync``)."""
         n = self.sizes[g]
-        f = np.zeros(2 * n)
+        f = np.empty(2 * n)
         self._check(self.lib.fa2cu_batch_forces(self.h, int(g), dptr(f)))
-        return f.reshape(2, n).T.copy()
+        return _rows(f, n)
 
     def speed(self, g: int) -> dict:
         st = np.zeros(4)

@@ -246,6 +246,15 @@ template <class R> struct Layout : LayoutBase {
 
     int alloc(bool want_tree)
     {
+        mem.planned([&] { take_buffers(want_tree); });
+        if (mem.failed) {
+            set_cuda_error("could not allocate memory on the device", mem.err);
+            return 1;
+        }
+        return 0;
+    }
+    void take_buffers(bool want_tree)
+    {
         const size_t nn = (size_t) n;
         pos = mem.get<R2>(nn);
         f = mem.get<R2>(nn);
@@ -295,11 +304,6 @@ template <class R> struct Layout : LayoutBase {
             packed = mem.get<typename ExactRec<R>::type>(nn);
             if (exact_nrows > 1) exact_part = mem.get<R2>((size_t) exact_nrows * nn);
         }
-        if (mem.failed) {
-            set_cuda_error("could not allocate memory on the device", mem.err);
-            return 1;
-        }
-        return 0;
     }
 
     // The graph from its edge list, prepared on the device (prep.cu): the
@@ -311,13 +315,18 @@ template <class R> struct Layout : LayoutBase {
         tmp.pool = mem.pool;
         tmp.s = s;
         const size_t m1 = (size_t) std::max(E.m, 1);
-        int *from = tmp.get<int>(m1), *to = tmp.get<int>(m1);
-        double *w = tmp.get<double>(m1);
-        double *dmass = tmp.get<double>((size_t) n);
-        int *dnode = tmp.get<int>(2 * m1);
-        double *dcoef = tmp.get<double>(std::max(2 * m1, (size_t) n));
+        int *from = nullptr, *to = nullptr, *dnode = nullptr;
+        double *w = nullptr, *dmass = nullptr, *dcoef = nullptr;
         PrepScratch ws;
-        prep_scratch(tmp, n, E.m, ws);
+        tmp.planned([&] {
+            from = tmp.get<int>(m1);
+            to = tmp.get<int>(m1);
+            w = tmp.get<double>(m1);
+            dmass = tmp.get<double>((size_t) n);
+            dnode = tmp.get<int>(2 * m1);
+            dcoef = tmp.get<double>(std::max(2 * m1, (size_t) n));
+            prep_scratch(tmp, n, E.m, ws);
+        });
         if (tmp.failed) {
             tmp.release();
             set_cuda_error("could not allocate memory on the device", tmp.err);
@@ -435,8 +444,12 @@ template <class R> struct Layout : LayoutBase {
             DevMem tmp;
             tmp.pool = mem.pool;
             tmp.s = s;
-            double *dd = tmp.get<double>(std::max<size_t>((size_t) n, (size_t) ninc));
-            int *di = tmp.get<int>((size_t) ninc);
+            double *dd = nullptr;
+            int *di = nullptr;
+            tmp.planned([&] {
+                dd = tmp.get<double>(std::max<size_t>((size_t) n, (size_t) ninc));
+                di = tmp.get<int>((size_t) ninc);
+            });
             if (tmp.failed) {
                 tmp.release();
                 set_cuda_error("could not allocate memory on the device", tmp.err);

@@ -75,24 +75,27 @@ def _flag(x, name):
 
 
 def _edges(n, edges):
-    e = np.asarray(edges if edges is not None else np.zeros((0, 2)), dtype=np.int64)
+    e = np.asarray(edges if edges is not None else np.zeros((0, 2)))
+    if e.dtype.kind not in "iu":
+        e = e.astype(np.int64)
     if e.size == 0:
         return np.zeros(0, np.int32), np.zeros(0, np.int32)
     if e.ndim != 2 or e.shape[1] != 2:
         raise ValueError("`edges` must be an (m, 2) array of 0-based node indices.")
-    if (e < 0).any() or (e >= n).any():
+    if e.min() < 0 or e.max() >= n:
         bad = int(np.flatnonzero(((e < 0) | (e >= n)).any(axis=1))[0])
         raise ValueError(f"edge {bad + 1} refers to a node that does not exist")
     if e.shape[0] > (1 << 30) - 1:
         raise ValueError("too many edges")
-    return e[:, 0].astype(np.int32), e[:, 1].astype(np.int32)
+    return (np.ascontiguousarray(e[:, 0], dtype=np.int32),
+            np.ascontiguousarray(e[:, 1], dtype=np.int32))
 
 
 def edge_weights(m, weights, edge_weight_influence=1.0, normalize_weights=False,
                  invert_weights=False):
     """Weights as the package transforms them (R/forceatlas2.R:254-264)."""
     if weights is None:
-        w = np.ones(m)
+        return np.ones(m)  # which every transformation leaves as they are
     else:
         try:
             w = np.asarray(weights, dtype=np.float64).reshape(-1)
@@ -112,7 +115,10 @@ def edge_weights(m, weights, edge_weight_influence=1.0, normalize_weights=False,
         lo, hi = w.min(), w.max()
         w = (w - lo) / (hi - lo) if lo < hi else np.ones(m)
     with np.errstate(over="ignore"):
-        w = np.ones(m) if edge_weight_influence == 0 else w ** edge_weight_influence
+        if edge_weight_influence == 0:
+            w = np.ones(m)
+        elif edge_weight_influence != 1:
+            w = w ** edge_weight_influence
     if (~np.isfinite(w)).any():
         raise ValueError("The edge weights are too large or too small to be used.")
     return w
@@ -250,9 +256,9 @@ class Layout:
         self._check(self.lib.fa2cu_layout_sync(self.h))
 
     def positions(self) -> np.ndarray:
-        xy = np.zeros(2 * self.n)
+        xy = np.empty(2 * self.n)
         self._check(self.lib.fa2cu_layout_positions(self.h, dptr(xy)))
-        return xy.reshape(2, self.n).T.copy()
+        return _rows(xy, self.n)
 
     def set_positions(self, pos):
         self._check(self.lib.fa2cu_layout_set_positions(
@@ -260,10 +266,10 @@ class Layout:
 
     def forces(self, pos) -> np.ndarray:
         """Forces of one iteration at pos (repulsion, gravity, attraction)."""
-        f = np.zeros(2 * self.n)
+        f = np.empty(2 * self.n)
         self._check(self.lib.fa2cu_layout_forces(self.h, dptr(_cols(pos, self.n)),
                                                  dptr(f)))
-        return f.reshape(2, self.n).T.copy()
+        return _rows(f, self.n)
 
     def speed(self):
         st = np.zeros(4)
@@ -342,15 +348,29 @@ class Layout:
             pass
 
 
-def _cols(pos, n):
-    """(n, 2) positions -> x then y (an R n x 2 matrix)."""
+def _positions(pos, n):
+    """(n, 2) finite positions."""
     pos = np.asarray(pos, dtype=np.float64)
     if pos.shape != (n, 2):
         raise ValueError(f"`init` must provide two numeric coordinates for each "
                          f"of the {n} nodes.")
-    if (~np.isfinite(pos)).any():
+    if not np.isfinite(pos).all():
         raise ValueError("`init` must not contain missing or infinite values.")
-    return np.ascontiguousarray(pos.T.reshape(-1))
+    return pos
+
+
+def _cols(pos, n):
+    """(n, 2) positions -> x then y (an R n x 2 matrix)."""
+    return np.ascontiguousarray(_positions(pos, n).T.reshape(-1))
+
+
+def _rows(xy, n):
+    """x then y -> (n, 2). Column by column: numpy copies a transposed (2, n)
+    array two values at a time (1,000,000 nodes: 3.1 ms against 1.1)."""
+    pos = np.empty((n, 2))
+    pos[:, 0] = xy[:n]
+    pos[:, 1] = xy[n:]
+    return pos
 
 
 def _resolve_device(device) -> int:
@@ -407,8 +427,7 @@ def _common(n, edges, iterations, scaling_ratio, gravity, jitter_tolerance,
         r = 10.0 * math.sqrt(n)
         pos = np.random.default_rng(seed).uniform(-r, r, size=(n, 2))
     else:
-        pos = np.asarray(init, dtype=np.float64)
-        _cols(pos, n)
+        pos = _positions(init, n)
     frm, to = _edges(n, edges)
     w = edge_weights(len(frm), weights, edge_weight_influence=edge_weight_influence,
                      normalize_weights=normalize_weights,
@@ -482,7 +501,7 @@ def layout_forceatlas2_large(n, edges, iterations=1000, scaling_ratio=None,
             int(dissuade_hubs), dptr(xy), dptr(t))
     if rc != 0:
         raise RuntimeError(_lib.error())
-    out = xy.reshape(2, n).T.copy()
+    out = _rows(xy, n)
     if timings:
         return out, dict(zip(FULL_TIME_NAMES, t))
     return out

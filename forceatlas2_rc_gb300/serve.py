@@ -16,7 +16,7 @@ import numpy as np
 
 from . import _lib
 from ._abi import ServerConfig, dptr
-from .layout import REPULSION_BH, Graph, _cols, _params
+from .layout import REPULSION_BH, Graph, _cols, _params, _rows
 
 
 def footprint(n: int, ninc: int, adjust: bool = False, any_fixed: bool = False,
@@ -84,14 +84,14 @@ class Server:
         if got < 0:
             raise RuntimeError(_lib.error())
         n = int(info[4])
-        buf = np.zeros(2 * n)
+        buf = np.empty(2 * n)
         if self.lib.fa2cu_server_collect(self.h, got, dptr(buf)) != 0:
             raise RuntimeError(f"job {got}: " + _lib.error())
         meta = dict(t_submit=info[0], t_resident=info[1], t_end=info[2],
                     n=n, iterations=int(info[5]), footprint=info[6],
                     speed=info[7], latency=info[2] - info[0],
                     queued=info[1] - info[0])
-        return got, buf.reshape(2, n).T.copy(), meta
+        return got, _rows(buf, n), meta
 
     def stats(self) -> dict:
         s = np.zeros(8)
