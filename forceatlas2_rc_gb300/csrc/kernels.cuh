@@ -846,6 +846,7 @@ __device__ __forceinline__ void climb(int k, int n, const typename RT<R>::R4 *ps
 
 } // namespace fa2cu
 
+#include "terms_walk.cuh"
 #include "tree.cuh"
 
 namespace fa2cu {

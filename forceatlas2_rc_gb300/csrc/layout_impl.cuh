@@ -173,7 +173,7 @@ template <class R> struct Layout : LayoutBase {
         tree_window = n < 60000 ? 64 : n < 400000 ? 32 : 16;
     }
     R scaling = 0, gravity = 0, theta2 = 0;
-    R wscale = 0; // FP32 records: size^2 (1 + DECIDE_BAND) / theta^2 (region_far)
+    R wscale = 0; // (1 + DECIDE_BAND) / theta^2 (region_far, term_bounds)
     double theta2d = 0.0;
     cudaStream_t s = nullptr;
     DevMem mem;
@@ -203,6 +203,7 @@ template <class R> struct Layout : LayoutBase {
     Agg<R> *agg = nullptr;
     R4 *rec_c = nullptr; // traversal records (common.cuh)
     int2 *rec_t = nullptr;
+    float4 *bounds = nullptr; // FP64: bounds of the opening tests (term_bounds)
     double2 *swing_partial = nullptr;
     SpeedState *st = nullptr;
     int *status = nullptr;
@@ -300,6 +301,7 @@ template <class R> struct Layout : LayoutBase {
             rec_c = mem.get<R4>(nn - 1);
             rec_t = mem.get<int2>(nn - 1);
             if (sizeof(R) == 4) fatt = mem.get<R2>(nn);
+            if (sizeof(R) == 8) bounds = mem.get<float4>(nn - 1);
         } else {
             packed = mem.get<typename ExactRec<R>::type>(nn);
             if (exact_nrows > 1) exact_part = mem.get<R2>((size_t) exact_nrows * nn);
@@ -570,8 +572,8 @@ template <class R> struct Layout : LayoutBase {
     }
     template <bool FULL> void launch_tree_kernel()
     {
-        const TreeArrays<R> A{psort, rec_c, child, range, rec_t, parent, rope, meet, agg, piece,
-                              pieces};
+        const TreeArrays<R> A{psort, rec_c, child, range, rec_t, parent, rope, meet, agg, bounds,
+                              piece, pieces};
         const int blocks = ceil_div(n, TREE_THREADS - 2 * tree_window);
         auto go = [&](auto kernel) {
             launch_k(pdl, kernel, dim3(blocks), dim3(TREE_THREADS), 0, s, n, tree_window, adjust,
@@ -610,14 +612,20 @@ template <class R> struct Layout : LayoutBase {
                         n, scaling, theta2, theta2d, psort, rec_c, rec_t, range, agg, rope, order, f,
                         status);
             } else if (walk == WALK_THREAD) {
-                if (adjust)
+                if constexpr (sizeof(R) == 8) {
+                    auto go = [&](auto kernel) {
+                        launch_k(pdl, kernel, dim3(ceil_div(n, 32 * TW_WARPS)),
+                                 dim3(32 * TW_WARPS), 0, s, n, scaling, theta2, psort, rec_c,
+                                 bounds, rec_t, rope, order, f, status);
+                    };
+                    adjust ? go(k_traverse_terms<true>) : go(k_traverse_terms<false>);
+                } else if (adjust) {
                     k_traverse<R, true, 6><<<ceil_div(n, 256), 256, 0, s>>>(
                         n, scaling, theta2, theta2d, psort, rec_c, rec_t, agg, rope, order, f, status);
-                else // float: 8 blocks per SM (0.597 against 0.619 ms at 6, 10^6 nodes)
-                    k_traverse<R, false, sizeof(R) == 4 ? 8 : 6>
-                        <<<ceil_div(n, 256), 256, 0, s>>>(n, scaling, theta2, theta2d, psort,
-                                                          rec_c, rec_t, agg, rope, order, f,
-                                                          status);
+                } else { // 8 blocks per SM (0.597 against 0.619 ms at 6, 10^6 nodes)
+                    k_traverse<R, false, 8><<<ceil_div(n, 256), 256, 0, s>>>(
+                        n, scaling, theta2, theta2d, psort, rec_c, rec_t, agg, rope, order, f, status);
+                }
             } else if (walk == WALK_DEFERRED) {
                 if constexpr (sizeof(R) == 4) {
                     launch_group_walk();

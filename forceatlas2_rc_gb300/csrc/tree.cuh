@@ -56,6 +56,7 @@ template <class R> struct TreeArrays {
     int2 *child, *range, *rec_t;
     int *parent, *rope, *meet;
     Agg<R> *agg;
+    float4 *bounds; // of the FP64 walk's opening tests (term_bounds)
     // the regions and leaves that climb (APART): TREE_PIECES places a block,
     // and how many
     int2 *piece;
@@ -73,7 +74,9 @@ __device__ __forceinline__ void write_region(const TreeArrays<R> &A, int n, int 
 {
     const int nl = n - 1;
     const int left = l == s ? nl + s : s, right = r == s + 1 ? nl + s + 1 : s + 1;
-    A.rec_c[idx] = agg_record(q, wscale);
+    const typename RT<R>::R4 rec = agg_record(q, wscale);
+    A.rec_c[idx] = rec;
+    if constexpr (sizeof(R) == 8) A.bounds[idx] = term_bounds(rec, wscale);
     // a region of at most 8 nodes is never opened: its left link carries its
     // packed range instead (negative)
     A.rec_t[idx] = make_int2(r - l >= 8 ? left : bucket_pack(l, r), after);
