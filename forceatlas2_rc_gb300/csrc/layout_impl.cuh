@@ -613,12 +613,17 @@ template <class R> struct Layout : LayoutBase {
                         status);
             } else if (walk == WALK_THREAD) {
                 if constexpr (sizeof(R) == 8) {
-                    auto go = [&](auto kernel) {
-                        launch_k(pdl, kernel, dim3(ceil_div(n, 32 * TW_WARPS)),
+                    auto go = [&](auto kernel, int nodes) {
+                        launch_k(pdl, kernel, dim3(ceil_div(n, nodes * TW_WARPS)),
                                  dim3(32 * TW_WARPS), 0, s, n, scaling, theta2, psort, rec_c,
                                  bounds, rec_t, rope, order, f, status);
                     };
-                    adjust ? go(k_traverse_terms<true>) : go(k_traverse_terms<false>);
+                    // (four nodes a warp while that does not fill the device)
+                    if (n < 12000)
+                        adjust ? go(k_traverse_terms<true, 4>, 4) : go(k_traverse_terms<false, 4>, 4);
+                    else
+                        adjust ? go(k_traverse_terms<true, 16>, 16)
+                               : go(k_traverse_terms<false, 16>, 16);
                 } else if (adjust) {
                     k_traverse<R, true, 6><<<ceil_div(n, 256), 256, 0, s>>>(
                         n, scaling, theta2, theta2d, psort, rec_c, rec_t, agg, rope, order, f, status);

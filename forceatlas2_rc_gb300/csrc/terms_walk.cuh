@@ -3,9 +3,9 @@
 
 namespace fa2cu {
 
-// A lane walks for each node, as walk() does: the same regions and nodes in
-// the same order, every force the same operations. Two things are done by the
-// warp instead:
+// NODES lanes of a warp walk, each for a node, as walk() does: the same regions
+// and nodes in the same order, every force the same operations. Two things are
+// done otherwise:
 //
 // - The opening test is made in float, against bounds on both sides of the
 //   region's boundary that hold for every rounding of the float coordinates
@@ -18,15 +18,22 @@ namespace fa2cu {
 // its result is 64 cycles away. walk() filled 14 of a warp's 32 lanes in them
 // -- lanes that add wait for lanes that test -- and a third of them were
 // tests; and 196 blocks of eight warps left most SMs idle while some had two
-// (50,021 nodes). The walk in us, walk() and this: 3,001 nodes 447 / 174;
-// 10,007 515 / 205; 50,021 1,083 / 325; 300,007 4,548 / 1,820.
+// (50,021 nodes).
+//
+// NODES: fewer make more warps and less waiting of one lane for another, and
+// more instructions of the walk and of the sums a node. The walk in us, walk()
+// and this with 32 / 16 / 8 / 4 nodes a warp: 1,000 nodes - and 145 / 102 / 85 /
+// 72; 3,001 447 and 173 / 125 / 104 / 88; 10,007 515 and 207 / 150 / 137 / 135;
+// 50,021 1,083 and 322 / 302 / 375 / 424; 300,007 4,548 and 1,827 / 1,791 /
+// 2,090 / 2,506. A large layout is bound by the FP64 pipe, a small one by the
+// serial chain of a lane's steps.
 constexpr int TW_WARPS = 2;      // a block
-constexpr int TW_POOL = 128;     // pairs evaluated at a time
+constexpr int TW_POOL = 128;     // pairs evaluated at a time (64 or 192: within 3 %)
 constexpr int TW_ROOM = TW_POOL + 32;
 
 struct TermsShared {
     double4 node[32];            // the lanes' nodes
-    double2 term[TW_POOL];
+    double term[2][TW_POOL];     // x and y
     int source[TW_ROOM];         // a region, or regions + node
     uint8_t owner[TW_ROOM];      // lane
     uint8_t next[TW_ROOM];       // the lane's next place in the pool
@@ -80,11 +87,12 @@ __device__ __forceinline__ void terms_eval(TermsShared &S, int count, int nl, do
         } else {
             g = d2 > 0.0 ? fdiv(scaling * mm, d2) : 0.0;
         }
-        S.term[t] = make_double2(xd * g, yd * g);
+        S.term[0][t] = xd * g;
+        S.term[1][t] = yd * g;
     }
 }
 
-template <bool ADJUST>
+template <bool ADJUST, int NODES>
 __global__ void __launch_bounds__(32 * TW_WARPS)
 k_traverse_terms(int n, double scaling, double theta2, const double4_32a *__restrict__ psort,
                  const double4_32a *__restrict__ rec_c, const float4 *__restrict__ bounds,
@@ -95,7 +103,8 @@ k_traverse_terms(int n, double scaling, double theta2, const double4_32a *__rest
     __shared__ TermsShared shared[TW_WARPS];
     TermsShared &S = shared[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int warp = blockIdx.x * TW_WARPS + (threadIdx.x >> 5);
+    const int k = lane < NODES ? warp * NODES + lane : n;
     const int nl = n - 1;
     unsigned below;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(below));
@@ -109,7 +118,7 @@ k_traverse_terms(int n, double scaling, double theta2, const double4_32a *__rest
     }
     __syncwarp();
     const float fx = (float) mx, fy = (float) my;
-    double ax = 0.0, ay = 0.0;
+    double sum = 0.0; // of the forces' x or y
     // (walk positions and the step limit as in walk())
     const unsigned nend = (unsigned) (nl + n);
     int cur = k < n ? 0 : -1, j = 0, jend = -1;
@@ -121,12 +130,15 @@ k_traverse_terms(int n, double scaling, double theta2, const double4_32a *__rest
         terms_eval<ADJUST>(S, count, nl, scaling, psort, rec_c);
         __syncwarp();
         const bool over = mine > 0 && tail >= count; // one at most, from the last step
-        int p = head;
-        for (int c = over ? 1 : 0; c < mine; c++) {
-            const double2 t = S.term[p];
+        // x by the node's lane, y by the one NODES above
+        const int from = lane % NODES;
+        int p = __shfl_sync(0xffffffffu, head, from);
+        int c = __shfl_sync(0xffffffffu, over ? mine - 1 : mine, from);
+        const double *term = S.term[lane / NODES & 1];
+        if (lane >= 2 * NODES) c = 0;
+        for (; c > 0; c--) {
+            sum += term[p];
             p = S.next[p];
-            ax += t.x;
-            ay += t.y;
         }
         int src = 0;
         if (over) src = S.source[tail];
@@ -193,7 +205,8 @@ k_traverse_terms(int n, double scaling, double theta2, const double4_32a *__rest
         if (filled >= TW_POOL) flush(TW_POOL);
     }
     if (filled) flush(filled);
-    if (k < n) f[order[k]] = make_double2(ax, ay);
+    const double other = __shfl_down_sync(0xffffffffu, sum, NODES);
+    if (k < n) f[order[k]] = make_double2(sum, other);
 }
 
 } // namespace fa2cu

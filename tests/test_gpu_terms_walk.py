@@ -24,7 +24,7 @@ def _positions(kind, n, rng):
 
 @pytest.mark.parametrize("adjust", [False, True])
 @pytest.mark.parametrize("kind", ["uniform", "far", "coincident", "grid", "scales"])
-@pytest.mark.parametrize("n", [2, 9, 31, 32, 33, 64, 65, 500, 5003])
+@pytest.mark.parametrize("n", [2, 9, 31, 32, 33, 64, 65, 500, 5003, 11999, 12001])
 def test_terms_walk_equals_thread_walk(gpu, n, kind, adjust):
     rng = np.random.default_rng(n)
     pos = _positions(kind, n, rng)
