@@ -1634,19 +1634,29 @@ __device__ __forceinline__ void neumaier(double &s, double &c, double v)
     s = t;
 }
 
-__device__ inline void update_speed_dev(SpeedState *st, double tsw, double ttr)
+// What the speed update needs of the number of nodes.
+struct SpeedTerms {
+    double est, min_jt, n2;
+};
+__device__ inline SpeedTerms speed_terms(int n)
+{
+    SpeedTerms t;
+    t.est = __dmul_rn(0.05, sqrt((double) n));
+    t.min_jt = sqrt(t.est);
+    t.n2 = __dmul_rn((double) n, (double) n);
+    return t;
+}
+
+__device__ inline void update_speed(SpeedState *st, const SpeedTerms &T, double tsw, double ttr)
 {
     double speed = st->speed, eff = st->efficiency;
     st->total_swinging = tsw;
     st->total_traction = ttr;
     if (!(tsw > 0)) return;
-    const int n = st->n;
-    const double jitter = st->jitter_tolerance;
-    const double est = __dmul_rn(0.05, sqrt((double) n));
-    const double min_jt = sqrt(est), max_jt = 10.0;
-    double jt = __ddiv_rn(__dmul_rn(est, ttr), __dmul_rn((double) n, (double) n));
+    const double jitter = st->jitter_tolerance, max_jt = 10.0;
+    double jt = __ddiv_rn(__dmul_rn(T.est, ttr), T.n2);
     if (jt > max_jt) jt = max_jt;
-    if (jt < min_jt) jt = min_jt;
+    if (jt < T.min_jt) jt = T.min_jt;
     jt = __dmul_rn(jt, jitter);
     if (tsw > __dmul_rn(2.0, ttr)) {
         if (eff > 0.05) eff = __dmul_rn(eff, 0.5);
@@ -1663,6 +1673,10 @@ __device__ inline void update_speed_dev(SpeedState *st, double tsw, double ttr)
     speed = __dadd_rn(speed, rise < cap ? rise : cap);
     st->speed = speed;
     st->efficiency = eff;
+}
+__device__ inline void update_speed_dev(SpeedState *st, double tsw, double ttr)
+{
+    update_speed(st, speed_terms(st->n), tsw, ttr);
 }
 
 // In the FP64 path, up to this many nodes the totals are summed serially in
@@ -1981,8 +1995,29 @@ k_add_forces(int n, const typename RT<R>::R2 *__restrict__ fa, typename RT<R>::R
 
 // ---- 8. displacement (pipeline.cl:476-506) ---------------------------------
 
-// The displacement (reference src/forceatlas2.c:780-802), fused with the
-// bounding box of the new positions that the next iteration's Morton codes
+// Where a node at p goes under force a (reference src/forceatlas2.c:780-802).
+template <class R>
+__device__ __forceinline__ typename RT<R>::R2 moved(typename RT<R>::R2 p, typename RT<R>::R2 a,
+                                                    R swinging, R speed, int adjust)
+{
+    R factor;
+    if (adjust) {
+        const R df = fsqrt(a.x * a.x + a.y * a.y);
+        factor = fdiv(R(0.1) * speed, R(1) + fsqrt(speed * swinging));
+        if (df > R(0)) {
+            if (factor * df > R(10)) factor = fdiv(R(10), df);
+        } else {
+            factor = R(0);
+        }
+    } else {
+        factor = fdiv(speed, R(1) + fsqrt(speed * swinging));
+    }
+    p.x += a.x * factor;
+    p.y += a.y * factor;
+    return p;
+}
+
+// The displacement of every node, fused with the bounding box of the new positions that the next iteration's Morton codes
 // need: a grid-stride pass (the bounding box's block count) that moves every
 // node that may move and folds every node's position into the block's
 // minima / maxima, then bbox_finish (skipped when partial is null: exact
@@ -2007,20 +2042,7 @@ k_apply(int n, int adjust, const typename RT<R>::R2 *__restrict__ f,
             const typename RT<R>::R2 a = f[i];
             fold[i] = a;
             if (!(fixed && fixed[i])) {
-                R factor;
-                if (adjust) {
-                    const R df = fsqrt(a.x * a.x + a.y * a.y);
-                    factor = fdiv(R(0.1) * speed, R(1) + fsqrt(speed * sw[i]));
-                    if (df > R(0)) {
-                        if (factor * df > R(10)) factor = fdiv(R(10), df);
-                    } else {
-                        factor = R(0);
-                    }
-                } else {
-                    factor = fdiv(speed, R(1) + fsqrt(speed * sw[i]));
-                }
-                p.x += a.x * factor;
-                p.y += a.y * factor;
+                p = moved<R>(p, a, sw[i], speed, adjust);
                 pos[i] = p;
                 if (rec) exact_move(rec + i, p); // the all-pairs kernel's record
             }
@@ -2159,6 +2181,35 @@ __device__ __forceinline__ void tma_load_1d(void *dst, const void *src, unsigned
         : "memory");
 }
 
+// The terms of a source (negated place, mass, radius; each twice) on two nodes
+// of radii sa, sb, without the nodes' scaling * mass, added to (ax, ay).
+// d2 carries 1e-30 (d2 = xd^2 + (yd^2 + 1e-30), one FMA each): a coincident
+// pair (xd = yd = 0) then has a finite factor below 1e30 m_j, so its term is 0
+// -- the reference's factor for d2 = 0 -- without a compare; any other pair of
+// float positions is at least ~1e-14 apart in d2 for coordinates of 1e-3 or
+// more, which the 1e-30 leaves unchanged to float precision.
+template <bool ADJUST>
+__device__ __forceinline__ void exact_term(const GroupNode &me, float sa, float sb, f2 nx, f2 ny,
+                                           f2 m, f2 r, f2 &ax, f2 &ay)
+{
+    const f2 xd = f2_add(me.x, nx), yd = f2_add(me.y, ny);
+    f2 g;
+    if (ADJUST) {
+        float d2a, d2b, ma, mb, ra, rb;
+        f2_split(f2_fma(xd, xd, f2_mul(yd, yd)), d2a, d2b);
+        f2_split(m, ma, mb);
+        f2_split(r, ra, rb);
+        const float da = fsqrt(d2a) - (sa + ra);
+        const float db = fsqrt(d2b) - (sb + rb);
+        g = f2_make(da > 0.0f ? ma * rcp_approx(da * da) : da < 0.0f ? 100.0f * ma : 0.0f,
+                    db > 0.0f ? mb * rcp_approx(db * db) : db < 0.0f ? 100.0f * mb : 0.0f);
+    } else {
+        g = pull2(m, f2_fma(xd, xd, f2_fma(yd, yd, f2_make(1e-30f, 1e-30f))));
+    }
+    ax = f2_fma(xd, g, ax);
+    ay = f2_fma(yd, g, ay);
+}
+
 // Block (x, y) sums, for its EXACT_THREADS * IPT nodes, the sources [y seg,
 // min(n, (y + 1) seg)) into row y of `partial` (n entries a row); the rows are
 // added in order by who reads them (exact_sum).
@@ -2208,7 +2259,6 @@ k_exact(int n, float scaling, const ExactF32 *__restrict__ nodes, float2 *__rest
                         cnt * (unsigned) sizeof(ExactF32), &bar[t]);
         }
     }
-    const f2 tiny = f2_make(1e-30f, 1e-30f);
     for (int t = 0; t < ntiles; t++) {
         const int b = t & 1;
         if (!mbar_wait(&bar[b], (t >> 1) & 1, 2000000000ull)) failed = 1;
@@ -2225,13 +2275,6 @@ k_exact(int n, float scaling, const ExactF32 *__restrict__ nodes, float2 *__rest
         }
         const int cnt = min(EXACT_TILE, j1 - j0 - t * EXACT_TILE);
         unsigned q = smem_addr(tile[b]);
-        // d2 carries 1e-30 (d2 = xd^2 + (yd^2 + 1e-30), one FMA each): a
-        // coincident pair (xd = yd = 0) then has a finite factor below 1e30
-        // m_j, so its term is 0 -- the reference's factor for d2 = 0 --
-        // without a compare; any other pair of float positions is at least
-        // ~1e-14 apart in d2 for coordinates of 1e-3 or more, which the 1e-30
-        // leaves unchanged to float precision. The thread's scaling * m_i
-        // multiplies the sums once at the end.
 #pragma unroll 4
         for (int jj = 0; jj < cnt; jj++, q += (unsigned) sizeof(ExactF32)) {
             f2 nx, ny, m, r;
@@ -2242,23 +2285,7 @@ k_exact(int n, float scaling, const ExactF32 *__restrict__ nodes, float2 *__rest
                 m = lds_1<16>(q);
 #pragma unroll
             for (int u = 0; u < P; u++) {
-                const f2 xd = f2_add(me[u].x, nx), yd = f2_add(me[u].y, ny);
-                f2 g;
-                if (ADJUST) {
-                    float d2a, d2b, ma, mb, ra, rb;
-                    f2_split(f2_fma(xd, xd, f2_mul(yd, yd)), d2a, d2b);
-                    f2_split(m, ma, mb);
-                    f2_split(r, ra, rb);
-                    const float da = fsqrt(d2a) - (si[2 * u] + ra);
-                    const float db = fsqrt(d2b) - (si[2 * u + 1] + rb);
-                    g = f2_make(
-                        da > 0.0f ? ma * rcp_approx(da * da) : da < 0.0f ? 100.0f * ma : 0.0f,
-                        db > 0.0f ? mb * rcp_approx(db * db) : db < 0.0f ? 100.0f * mb : 0.0f);
-                } else {
-                    g = pull2(m, f2_fma(xd, xd, f2_fma(yd, yd, tiny)));
-                }
-                ax[u] = f2_fma(xd, g, ax[u]);
-                ay[u] = f2_fma(yd, g, ay[u]);
+                exact_term<ADJUST>(me[u], si[2 * u], si[2 * u + 1], nx, ny, m, r, ax[u], ay[u]);
             }
         }
         __syncthreads(); // every thread is done with buffer b
@@ -2462,3 +2489,5 @@ k_qtraverse(int n, R scaling, R theta2, double theta2d, const typename RT<R>::R4
 }
 
 } // namespace fa2cu
+
+#include "small_exact.cuh"

@@ -134,28 +134,37 @@ template <class R> struct Layout : LayoutBase {
     static bool cluster_fits(int n, int c, int shape)
     {
         if (c < 1 || c > CS_MAX_BLOCKS || ceil_div(n, c) > cluster_pairs[shape]) return false;
-        int fit = 0;
+        bool fit = false;
         with_cluster_kernel(shape, [&](auto kernel, int threads) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned) c);
-            cfg.blockDim = dim3((unsigned) threads);
-            cfg.dynamicSmemBytes = 2 * sizeof(uint2) * (size_t) ceil_div(n, c);
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = (unsigned) c;
-            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     2 * (int) sizeof(uint2) * cluster_pairs[shape]) !=
-                    cudaSuccess ||
-                cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-                    cudaSuccess ||
-                cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) != cudaSuccess) {
-                cudaGetLastError();
-                fit = 0;
-            }
+            fit = cluster_runs(kernel, c, threads, 2 * sizeof(uint2) * (size_t) ceil_div(n, c),
+                               2 * sizeof(uint2) * (size_t) cluster_pairs[shape]);
         });
+        return fit;
+    }
+    // Whether a cluster of c blocks of the kernel runs on the current device
+    // with smem bytes of dynamic shared memory a block (at most `most`, which
+    // the kernel is allowed).
+    template <class K> static bool cluster_runs(K kernel, int c, int threads, size_t smem, size_t most)
+    {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned) c);
+        cfg.blockDim = dim3((unsigned) threads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned) c;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int fit = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int) most) != cudaSuccess ||
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+                cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
         return fit > 0;
     }
 
@@ -171,6 +180,25 @@ template <class R> struct Layout : LayoutBase {
     {
         tree_apart = n >= 400000;
         tree_window = n < 60000 ? 64 : n < 400000 ? 32 : 16;
+    }
+    // FP32 all-pairs: blocks of the cluster that runs whole iterations
+    // (k_small_exact; 0: three launches an iteration)
+    int small_blocks = 0;
+    bool pick_small(int c)
+    {
+        if constexpr (sizeof(R) == 4) {
+            if (repulsion != FA2CU_REPULSION_EXACT || nheavy > 0 || c < 1 || c > CS_MAX_BLOCKS ||
+                ceil_div(n, c) > SE_THREADS || small_exact_smem(n) > SE_SMEM)
+                return false;
+            auto runs = [&](auto kernel) {
+                return cluster_runs(kernel, c, SE_THREADS, small_exact_smem(n), SE_SMEM);
+            };
+            if (adjust ? runs(k_small_exact<true>) : runs(k_small_exact<false>)) {
+                small_blocks = c;
+                return true;
+            }
+        }
+        return false;
     }
     R scaling = 0, gravity = 0, theta2 = 0;
     R wscale = 0; // (1 + DECIDE_BAND) / theta^2 (region_far, term_bounds)
@@ -516,9 +544,8 @@ template <class R> struct Layout : LayoutBase {
         h.n = n;
         FA2_TRY(cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, s), "cudaMemcpy", 1);
         FA2_TRY(cudaStreamSynchronize(s), "could not prepare the layout", 1);
-        if (capture(&g1, 1)) return 1;
-        if (n <= (1 << 16) && capture(&g8, 8)) return 1;
-        return 0;
+        if (n <= SE_MAX) pick_small(n <= 200 ? 1 : CS_MAX_BLOCKS);
+        return make_graphs();
     }
 
     static int exact_layout_rows(int n, int sms)
@@ -839,12 +866,33 @@ template <class R> struct Layout : LayoutBase {
     int iterate(int iterations) override
     {
         cudaSetDevice(device);
+        if constexpr (sizeof(R) == 4) {
+            if (small_blocks) return iterate_small(iterations);
+        }
         while (iterations >= 8 && g8) {
             FA2_TRY(cudaGraphLaunch(g8, s), "the computation on the GPU failed", 1);
             iterations -= 8;
         }
         for (; iterations > 0; iterations--)
             FA2_TRY(cudaGraphLaunch(g1, s), "the computation on the GPU failed", 1);
+        return 0;
+    }
+
+    // (a launch's iterations are bounded: other work may wait for the SMs)
+    int iterate_small(int iterations)
+    {
+        for (; iterations > 0; iterations -= SE_ITERATIONS) {
+            auto go = [&](auto kernel) {
+                return launch_cluster(small_blocks, pdl, kernel, dim3(small_blocks),
+                                      dim3(SE_THREADS), small_exact_smem(n), s, n,
+                                      ceil_div(n, small_blocks),
+                                      std::min(iterations, SE_ITERATIONS), scaling, gravity,
+                                      strong, linlog, mass, size, fixed, inc_off, inc, pos, fold,
+                                      sw, trac, packed, st, status);
+            };
+            FA2_TRY(adjust ? go(k_small_exact<true>) : go(k_small_exact<false>),
+                    "the computation on the GPU failed", 1);
+        }
         return 0;
     }
 
@@ -1007,6 +1055,14 @@ template <class R> struct Layout : LayoutBase {
         if (g1) cudaGraphExecDestroy(g1);
         if (g8) cudaGraphExecDestroy(g8);
         g1 = g8 = nullptr;
+        return make_graphs();
+    }
+    int make_graphs()
+    {
+        if (small_blocks) { // (nothing to capture)
+            launches = 1;
+            return 0;
+        }
         if (capture(&g1, 1)) return 1;
         if (n <= (1 << 16) && capture(&g8, 8)) return 1;
         return 0;
@@ -1026,6 +1082,15 @@ template <class R> struct Layout : LayoutBase {
                 return 1;
             }
             cluster = c;
+            return recapture();
+        }
+        if (!strcmp(name, "exact_cluster") && value >= 0 && value <= CS_MAX_BLOCKS &&
+            value == (int) value) {
+            if (value != 0 && !pick_small((int) value)) {
+                set_message("a cluster of %d blocks does not run this layout", (int) value);
+                return 1;
+            }
+            small_blocks = (int) value;
             return recapture();
         }
         if (!strcmp(name, "sort_threads") && (value == 256 || value == 512 || value == 1024)) {

@@ -32,7 +32,7 @@ constexpr int TW_POOL = 128;     // pairs evaluated at a time (64 or 192: within
 constexpr int TW_ROOM = TW_POOL + 32;
 
 struct TermsShared {
-    double4 node[32];            // the lanes' nodes
+    double4_32a node[32];        // the lanes' nodes
     double term[2][TW_POOL];     // x and y
     int source[TW_ROOM];         // a region, or regions + node
     uint8_t owner[TW_ROOM];      // lane
@@ -72,7 +72,7 @@ __device__ __forceinline__ void terms_eval(TermsShared &S, int count, int nl, do
         const int src = S.source[t];
         const bool region = src < nl;
         const double4_32a q = region ? rec_c[src] : psort[src - nl];
-        const double4 me = S.node[S.owner[t]];
+        const double4_32a me = S.node[S.owner[t]];
         const double xd = me.x - q.x, yd = me.y - q.y;
         const double d2 = sq_dist(xd, yd), mm = me.z * q.z;
         // (a far region has d2 > 0)
@@ -112,7 +112,7 @@ k_traverse_terms(int n, double scaling, double theta2, const double4_32a *__rest
     double mx = 0.0, my = 0.0; // the node
     if (k < n) {
         const double4_32a me = psort[k];
-        S.node[lane] = make_double4(me.x, me.y, me.z, me.w);
+        S.node[lane] = me;
         mx = me.x;
         my = me.y;
     }

@@ -96,6 +96,11 @@ int fa2cu_layout_traversal_counts(fa2cu_layout *L, double counts[2]);
  *   "climb"        1: the tree in one launch; 2, 4, 8, -2 or -4: the regions
  *                  that span its blocks in a second one (default from
  *                  400,000 nodes; the same tree);
+ *   "exact_cluster" single precision, exact repulsion, no node of 128
+ *                  incidences or more: thread blocks of the cluster that runs
+ *                  whole iterations in one launch (1 .. 16, of 512 nodes at
+ *                  most each), 0 for three launches an iteration (default: 1
+ *                  up to 200 nodes, 16 up to 1,500, else 0)
  *   "sort_cluster" blocks (1 to 16) of the cluster that makes the codes and
  *                  sorts them in one launch (default: 1, 4 or 16 up to
  *                  110,000 nodes); 0: separate launches;
