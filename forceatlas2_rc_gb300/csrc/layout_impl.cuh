@@ -184,6 +184,13 @@ template <class R> struct Layout : LayoutBase {
     // FP32 all-pairs: blocks of the cluster that runs whole iterations
     // (k_small_exact; 0: three launches an iteration)
     int small_blocks = 0;
+    // Threads a block of the kernels with a thread a node that end in totals:
+    // small blocks spread a small layout over the SMs and have fewer warps to
+    // add up. An iteration in us with 256 / 128 / 64: all pairs FP32 1,600
+    // nodes 19.5 / 17.4 / 16.4, 6,007 30.4 / 28.5 / 27.7; Barnes-Hut FP32 3,001
+    // 57.9 / 56.1 / 55.3, 10,007 66.5 / 64.5 / 64.7, 30,011 84.4 / 82.8 / 85.7;
+    // FP64 3,001 155 / 146 / 143, 30,011 305 / 301 / 304.
+    int node_threads() const { return n < 20000 ? 64 : n < 200000 ? 128 : 256; }
     bool pick_small(int c)
     {
         if constexpr (sizeof(R) == 4) {
@@ -299,13 +306,13 @@ template <class R> struct Layout : LayoutBase {
             heavy_cap = ninc / HEAVY_DEGREE;
             heavy = mem.get<int>((size_t) heavy_cap + 1);
         }
-        swing_partial = mem.get<double2>((size_t) ceil_div(n, 256)); // one per block
+        swing_partial = mem.get<double2>((size_t) ceil_div(n, node_threads())); // one per block
         st = mem.get<SpeedState>(1);
         status = mem.get<int>(ST_COUNT);
         xy = mem.get<double>(2 * nn);
         counts = mem.get<unsigned long long>(2);
         if (want_tree) {
-            nbbox = std::min(ceil_div(n, 256), 152 * 4);
+            nbbox = std::min(ceil_div(n, node_threads()), 152 * 4);
             bbox = mem.get<R>(4);
             quant = mem.get<double>(6);
             bbox_partial = mem.get<R>(4 * (size_t) nbbox);
@@ -734,8 +741,8 @@ template <class R> struct Layout : LayoutBase {
             repulsion == FA2CU_REPULSION_EXACT && exact_nrows > 1 && nheavy == 0;
         if (!in_rows) launch_exact_sum();
         launch_heavy();
-        launch_k(pdl && nheavy == 0, k_attract_swing<R>, dim3(ceil_div(n, 256)), dim3(256), smem,
-                 s, n, gravity, strong, linlog, adjust, in_rows ? exact_nrows : 0, exact_part,
+        launch_k(pdl && nheavy == 0, k_attract_swing<R>, dim3(ceil_div(n, node_threads())),
+                 dim3(node_threads()), smem, s, n, gravity, strong, linlog, adjust, in_rows ? exact_nrows : 0, exact_part,
                  pos, mass, size, inc_off, inc, f, fold, fixed, sw, trac, swing_partial,
                  (unsigned *) (status + ST_TICKET_SWING), st, status);
     }
@@ -744,9 +751,9 @@ template <class R> struct Layout : LayoutBase {
     {
         // with a tree, the bounding box's block count (its partials); else
         // one thread per node
-        const int nb = bbox_partial ? nbbox : ceil_div(n, 256);
-        launch_k(pdl, k_apply<R>, dim3(nb), dim3(256), 0, s, n, adjust, f, fold, sw, fixed, pos,
-                 st, status, bbox_partial, bbox, quant, (unsigned *) (status + ST_TICKET_BBOX),
+        const int nb = bbox_partial ? nbbox : ceil_div(n, node_threads());
+        launch_k(pdl, k_apply<R>, dim3(nb), dim3(node_threads()), 0, s, n, adjust, f, fold, sw,
+                 fixed, pos, st, status, bbox_partial, bbox, quant, (unsigned *) (status + ST_TICKET_BBOX),
                  packed);
     }
     void launch_repel()
@@ -798,7 +805,8 @@ template <class R> struct Layout : LayoutBase {
     }
     void launch_join_swing()
     {
-        k_join_swing<R><<<std::min(ceil_div(n, 256), join_blocks), 256, 0, s>>>(
+        const int nb = std::min(ceil_div(n, node_threads()), join_blocks);
+        k_join_swing<R><<<nb, node_threads(), 0, s>>>(
             n, fatt, f, fold, mass, fixed, sw, trac, swing_partial,
             (unsigned *) (status + ST_TICKET_SWING), st, status);
     }
