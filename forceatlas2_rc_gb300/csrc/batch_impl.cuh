@@ -410,15 +410,16 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
             double ttr = block_sum<W>(tt, red2);
             if (serial) {
                 __syncthreads(); // sw / tr written by every thread
-                if (tid == 0) {
-                    tsw = 0.0;
-                    ttr = 0.0;
-                    for (int i = 0; i < n; i++) {
-                        if (fixed && fixed[i]) continue;
-                        tsw = __dadd_rn(tsw, (double) sw[i]);
-                        ttr = __dadd_rn(ttr, (double) tr[i]);
-                    }
+                if (tid < 64) { // a warp each
+                    const R *v = tid < 32 ? sw : tr;
+                    const double sum = ordered_sum(n, [&](int i) {
+                        return fixed && fixed[i] ? 0.0 : (double) v[i];
+                    });
+                    if ((tid & 31) == 0) red[tid >> 5] = sum;
                 }
+                __syncthreads();
+                tsw = red[0];
+                ttr = red[1];
             }
             if (tid == 0) {
                 if (!(tsw == tsw) || !(ttr == ttr)) {

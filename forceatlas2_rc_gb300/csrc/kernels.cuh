@@ -1525,6 +1525,92 @@ __device__ __forceinline__ void attract_one(int i, R gravity, int strong, int li
     f[i] = mk2<R>(ax, ay);
 }
 
+// The same for the FP64 path, by a whole warp, a lane a node (`have`: the
+// lane's node exists): the terms, which attract_one makes, are evaluated with
+// the lanes spread evenly over the incidences that are left, 128 at a time, and
+// each lane adds up its own in edge order.
+//
+// Why: a hub's lane walked through its incidences alone, a thousand cycles for
+// four (an FP64 instruction's result is 64 cycles away), and the warp with it.
+// The attraction with the totals of 1,500 nodes, preferential attachment: 109 ->
+// 78 us. Without hubs (up to 32 incidences) the lanes alone are as fast or
+// faster (3,001 nodes 22 against 31 us).
+constexpr int AW_TERMS = 128;
+constexpr int AW_HUB = 32; // a warp without a node of more incidences takes them lane by lane
+struct AttractShared {
+    double x[32], y[32], r[32];   // the lanes' nodes
+    double tx[AW_TERMS], ty[AW_TERMS];
+    int first[32];                // a lane's next incidence, less its first place
+    uint8_t owner[AW_TERMS];      // lane
+};
+static __device__ __forceinline__ void
+attract_warp(AttractShared &S, bool have, int i, double gravity, int strong, int linlog,
+             int adjust, const double2 *pos, const double *mass, const double *size,
+             const int *off, const Inc<double> *inc, double2 *f)
+{
+    const int lane = threadIdx.x & 31;
+    double ax = 0.0, ay = 0.0;
+    int e = 0, e1 = 0;
+    if (have) {
+        const double2 p = pos[i], a = f[i];
+        ax = a.x;
+        ay = a.y;
+        if (gravity != 0.0) {
+            const double dist = fsqrt(p.x * p.x + p.y * p.y);
+            if (dist > 0.0) {
+                const double g = strong ? gravity * mass[i] : fdiv(gravity * mass[i], dist);
+                ax -= p.x * g;
+                ay -= p.y * g;
+            }
+        }
+        e = off[i];
+        e1 = off[i + 1];
+        S.x[lane] = p.x;
+        S.y[lane] = p.y;
+        S.r[lane] = adjust ? size[i] : 0.0;
+    }
+    for (;;) {
+        const unsigned active = __ballot_sync(0xffffffffu, e < e1);
+        if (!active) break;
+        const int count = min(e1 - e, AW_TERMS / __popc(active));
+        int end = count;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += t;
+        }
+        const int total = __shfl_sync(0xffffffffu, end, 31), start = end - count;
+        S.first[lane] = e - start;
+        for (int q = start; q < end; q++) S.owner[q] = (uint8_t) lane;
+        __syncwarp();
+#pragma unroll 4
+        for (int t = lane; t < total; t += 32) {
+            const int o = S.owner[t];
+            const Inc<double> c = load_inc(inc + (S.first[o] + t));
+            const double2 q = pos[c.j];
+            const double xd = S.x[o] - q.x, yd = S.y[o] - q.y;
+            double g = -c.coef;
+            bool none = false;
+            if (adjust || linlog) {
+                double dist = fsqrt(xd * xd + yd * yd);
+                if (adjust) dist -= S.r[o] + size[c.j];
+                none = !(dist > 0.0);
+                if (linlog && !none) g *= fdiv(flog1p(dist), dist);
+            }
+            S.tx[t] = none ? -0.0 : xd * g; // (-0 added leaves any sum as it is)
+            S.ty[t] = none ? -0.0 : yd * g;
+        }
+        __syncwarp();
+        for (int q = start; q < end; q++) {
+            ax += S.tx[q];
+            ay += S.ty[q];
+        }
+        e += count;
+        __syncwarp();
+    }
+    if (have) f[i] = make_double2(ax, ay);
+}
+
 template <class R>
 __global__ void __launch_bounds__(256)
 k_attract(int n, R gravity, int strong, int linlog, int adjust,
@@ -1684,12 +1770,81 @@ __device__ inline void update_speed_dev(SpeedState *st, double tsw, double ttr)
 // hence the whole trajectory, is then the reference's bit for bit. Beyond,
 // and always in the FP32 path (whose forces differ from the reference's in
 // any case), a fixed-order tree: float-float in FP32, with compensation in
-// FP64. A serial chain of double additions costs about 70 ns an addition
-// on a GB300 (0.28 ms an iteration at 2000 nodes).
+// FP64.
 constexpr int SERIAL_TOTALS_MAX = 2048;
 template <class R> __host__ __device__ constexpr bool serial_totals(int n)
 {
     return sizeof(R) == 8 && n <= SERIAL_TOTALS_MAX;
+}
+
+// v(0) + v(1) + ... + v(n - 1), none negative, added to 0 in that order and
+// rounded after each addition: the bits of the serial sum, by a whole warp
+// (every lane gets it).
+//
+// While the sum s stays in one binade its roundings are to one spacing u, and s
+// is a multiple of u: fl(s + v) = s + (v rounded to a multiple of u), unless v
+// lies half-way between two. So 128 values are rounded alone and their prefix
+// sums taken, in integers that count the u's. The first value that is half-way,
+// that takes s out of the binade, or that is half of the binade's lower end or
+// more is added by an addition.
+//
+// Why: a dependent FP64 addition takes 64 cycles. The attraction with the
+// totals of 1,500 nodes (both sums, and their staging): 88 us serially, 40 with
+// this; of 300, 33 and 27. (The rounding by FP64 additions instead: 56.)
+template <class F> __device__ inline double ordered_sum(int n, F v)
+{
+    const int lane = threadIdx.x & 31;
+    constexpr long long MANT = (1LL << 52) - 1;
+    double s = 0.0;
+    for (int i = 0; i < n;) {
+        const long long bits = __double_as_longlong(s);
+        const long long E = bits >> 52; // (s >= 0, or not a number)
+        if (E < 64 || E > 2000) {       // tiny, or no finite sum
+            s = __dadd_rn(s, v(i));
+            i++;
+            continue;
+        }
+        // four values a lane, in order
+        double x[4];
+        long long r[4];
+        unsigned odd = 0;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int k = i + 4 * lane + q;
+            x[q] = k < n ? v(k) : 0.0;
+            const long long b = __double_as_longlong(x[q]), e = b >> 52;
+            const long long m = (b & MANT) | (e ? 1LL << 52 : 0);
+            // m shifted to the spacing of s, rounded to nearest
+            const int d = (int) min(E - e, 62LL);
+            const long long half = 1LL << (d > 0 ? d - 1 : 0), rest = m & (2 * half - 1);
+            r[q] = (m >> (d > 0 ? d : 0)) + (rest > half) + (q ? r[q - 1] : 0);
+            if (d < 2 || rest == half) odd |= 1u << q;
+        }
+        long long sum = r[3];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long t = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += t;
+        }
+        const long long before = sum - r[3] + ((bits & MANT) | (1LL << 52)); // of the lane's four
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (before + r[q] >= (1LL << 53)) odd |= 1u << q;
+        // (what a lane counts behind the first such value is not used)
+        const unsigned stop = __ballot_sync(0xffffffffu, odd != 0);
+        if (!stop) {
+            s = __longlong_as_double((E << 52) | (__shfl_sync(0xffffffffu, before + r[3], 31) & MANT));
+            i += 128;
+        } else {
+            const int j = __ffs(stop) - 1, q = __ffs(odd) - 1;
+            const long long mine = before + (q == 1 ? r[0] : q == 2 ? r[1] : q == 3 ? r[2] : 0);
+            const double next = q <= 0 ? x[0] : q == 1 ? x[1] : q == 2 ? x[2] : x[3];
+            s = __longlong_as_double((E << 52) | (__shfl_sync(0xffffffffu, mine, j) & MANT));
+            s = __dadd_rn(s, __shfl_sync(0xffffffffu, next, j));
+            i += 4 * j + __shfl_sync(0xffffffffu, q, j) + 1;
+        }
+    }
+    return s;
 }
 
 // Per-thread sums of swinging and traction over the nodes that can move:
@@ -1822,27 +1977,25 @@ __device__ __forceinline__ void swing_finish(SwingAcc<R> acc, int n, const uint8
     if (serial_totals<R>(n)) {
         // the block stages the nodes' values in shared memory (dynamic, 2n
         // reals; a fixed node's as +0, which leaves a sum unchanged), then
-        // one thread adds them in node order: the chain waits on the adds
-        // only, not on a load per node
+        // they are added in node order
         extern __shared__ __align__(16) unsigned char serial_smem[];
         R *ssw = reinterpret_cast<R *>(serial_smem), *str = ssw + n;
+#pragma unroll 4
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
             const bool skip = fixed && fixed[i];
             ssw[i] = skip ? R(0) : __ldcg(sw + i);
             str[i] = skip ? R(0) : __ldcg(tr + i);
         }
         __syncthreads();
-        // one lane sums the swinging, another the traction: an add of a
-        // warp's two lanes costs what one lane's does (64 cycles a dependent
-        // FP64 add)
-        if (threadIdx.x < 2) {
-            const R *v = threadIdx.x == 0 ? ssw : str;
-            double s = 0.0;
-#pragma unroll 8
-            for (int i = 0; i < n; i++) s = __dadd_rn(s, (double) v[i]);
-            tsw = s;
-            ttr = __shfl_down_sync(3u, s, 1);
+        // one warp sums the swinging, another the traction
+        if (w < 2) {
+            const R *v = w == 0 ? ssw : str;
+            const double sum = ordered_sum(n, [&](int i) { return (double) v[i]; });
+            if (lane == 0) ss[w] = sum;
         }
+        __syncthreads();
+        tsw = ss[0];
+        ttr = ss[1];
     } else if constexpr (sizeof(R) == 4) {
         // the partials per thread (strided, fixed order) and per warp in
         // float-float, whose same-sign sums lose about 2^-47 relative a step
@@ -1928,13 +2081,20 @@ k_attract_swing(int n, R gravity, int strong, int linlog, int adjust, int rows,
     pdl_wait();
     SwingAcc<R> acc;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        // the all-pairs repulsion still in rows (not yet in f)
-        if (rows > 0) f[i] = exact_sum<R>(i, n, rows, partial_f);
-        attract_one<R, sizeof(R) == 4>(i, gravity, strong, linlog, adjust, pos, mass, size, off,
-                                       inc, f);
-        swing_node<R>(i, n, f, fold, mass, fixed, sw, tr, acc);
+    if (i < n && rows > 0) f[i] = exact_sum<R>(i, n, rows, partial_f); // (not yet in f)
+    if constexpr (sizeof(R) == 8) {
+        extern __shared__ __align__(16) unsigned char serial_smem[]; // (then the totals')
+        const bool hub = i < n && off[i + 1] - off[i] > AW_HUB;
+        if (!__any_sync(0xffffffffu, hub)) {
+            if (i < n)
+                attract_one<R>(i, gravity, strong, linlog, adjust, pos, mass, size, off, inc, f);
+        } else
+            attract_warp(reinterpret_cast<AttractShared *>(serial_smem)[threadIdx.x >> 5], i < n, i,
+                     gravity, strong, linlog, adjust, pos, mass, size, off, inc, f);
+    } else if (i < n) {
+        attract_one<R, true>(i, gravity, strong, linlog, adjust, pos, mass, size, off, inc, f);
     }
+    if (i < n) swing_node<R>(i, n, f, fold, mass, fixed, sw, tr, acc);
     swing_finish<R>(acc, n, fixed, sw, tr, partial, ticket, st, status);
 }
 

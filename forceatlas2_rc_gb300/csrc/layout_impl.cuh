@@ -740,8 +740,10 @@ template <class R> struct Layout : LayoutBase {
     // update (an iteration's second half before the displacement).
     void launch_attraction_swing()
     {
-        // serial totals: the last block stages 2n reals
-        const size_t smem = serial_totals<R>(n) ? 2 * (size_t) n * sizeof(R) : 0;
+        // FP64: the warps' terms; serial totals: the last block stages 2n reals
+        size_t smem = serial_totals<R>(n) ? 2 * (size_t) n * sizeof(R) : 0;
+        if (sizeof(R) == 8)
+            smem = std::max(smem, node_threads() / 32 * sizeof(AttractShared));
         // the rows of the all-pairs sum are added up in the same launch,
         // unless a hub's attraction is added to them first
         const bool in_rows =
