@@ -55,8 +55,8 @@ WORKLOAD = ("SBM n=1,000,000, 1000 power-law blocks (exp 2.1), deg_in 12, "
             "deg_out 2, unit weights; linlog + dissuade_hubs, Barnes-Hut "
             "theta 1.2, FP32 positions/forces, FP64 speed control")
 # Barnes-Hut walks (fa2cu_layout_option "walk"): the same regions and node
-# pairs (the deferred walk adds them up in another order)
-WALKS = {"warp": 0, "thread": 1, "wide": 2, "pair": 3, "quad": 4, "deferred": 5}
+# pairs (the group walk adds them up in another order)
+WALKS = {"warp": 0, "thread": 1, "wide": 2, "pair": 3, "quad": 4, "group": 5}
 # algorithmic HBM bytes per node of the traversal: psort record 16, order 4,
 # force write 8 (FP32)
 TRAVERSE_HBM_BYTES_PER_NODE = 28
@@ -67,10 +67,10 @@ TRAVERSE_L2_BYTES_PER_PAIR = 16
 # DRAM bytes (read + write) of one traversal launch on this workload
 # (dram__bytes_read.sum + dram__bytes_write.sum, one ncu capture of each
 # walk), and the share of cycles the schedulers issued (the kernel's bound)
-TRAVERSE_DRAM_BYTES = {"deferred": 53.06e6 + 4.54e6, "thread": 45.94e6 + 0.86e6}
-TRAVERSE_ISSUE_ACTIVE = {"deferred": 0.757, "thread": 0.805}
+TRAVERSE_DRAM_BYTES = {"group": 53.88e6 + 1.61e6, "thread": 45.94e6 + 0.86e6}
+TRAVERSE_ISSUE_ACTIVE = {"group": 0.674, "thread": 0.805}
 # and its L1 throughput (share of peak, same captures)
-TRAVERSE_L1_THROUGHPUT = {"deferred": 0.859, "thread": 0.78}
+TRAVERSE_L1_THROUGHPUT = {"group": 0.737, "thread": 0.78}
 
 
 def make_workload(small: bool = False):
@@ -1146,9 +1146,10 @@ def headline(args, local, ws, pg):
                 "traffic": TRAVERSE_DRAM_BYTES.get(args.walk) if n == 1_000_000 else None,
                 "issue_active": TRAVERSE_ISSUE_ACTIVE.get(args.walk),
                 "l1_throughput": TRAVERSE_L1_THROUGHPUT.get(args.walk),
-                "bound_note": "L1- and issue-bound (ncu: L1 throughput ~86 % of peak, issue "
-                              "active ~76 %, 95 % L1 hits); the HBM fraction is small by "
-                              "design",
+                "bound_note": "L1- and issue-bound (ncu: L1 throughput ~74 % of peak, issue "
+                              "active ~67 %); the HBM fraction is small by design. "
+                              "l2_request_bytes counts what a walk per node asks for; "
+                              "the 32 nodes of a warp share most of it",
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of "
                                   "one traversal launch on this workload",
                 "kernel": {"warp": "k_traverse_warp<float, 0>",
@@ -1156,7 +1157,7 @@ def headline(args, local, ws, pg):
                            "wide": "k_traverse<float, 0, 1>",
                            "pair": "k_traverse_multi<float, 0, 2>",
                            "quad": "k_traverse_multi<float, 0, 4>",
-                           "deferred": "k_traverse_deferred<float, 0, 8>"}[args.walk],
+                           "group": "k_traverse_group<0, 0>"}[args.walk],
                 "peak_kind": f"{kind} (HBM copy)",
                 "launch_ms": ph["repulsion"],
                 "l2_request_bytes": l2_bytes,
@@ -1211,9 +1212,9 @@ def main():
                          "kernel alone on 100,000 nodes (FP32 pipe figures); "
                          "batch: 4096 graphs in one persistent launch; "
                          "serve: the layout server on a Poisson job trace")
-    ap.add_argument("--walk", default="deferred",
+    ap.add_argument("--walk", default="group",
                     choices=list(WALKS),
-                    help="Barnes-Hut walk (the same interactions; deferred is the "
+                    help="Barnes-Hut walk (the same interactions; group is the "
                          "FP32 default)")
     args = ap.parse_args()
     if args.impl == "reference":
