@@ -320,7 +320,7 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
                     psort[k] = mk4<R>(p.x, p.y, mass[i], adjust ? size[i] : R(0));
                 }
                 for (int i = tid; i < n - 1; i += T)
-                    karras_one<false>(i, n, key, child, range, parent, rope, visits);
+                    karras_one(i, n, key, child, range, parent, rope, visits);
                 __syncthreads();
                 phase(BP_TREE);
                 // contiguous leaves per thread: a thread's later climbs find

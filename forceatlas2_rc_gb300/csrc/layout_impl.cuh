@@ -11,10 +11,12 @@
 //   psort               R4[n]   (x, y, m, r) in Morton order
 //   child, range        int2[n-1], parent int[2n-1], rope int[n],
 //   meet                int[n-1], agg Agg<R>[n-1] (double / float-float sums),
-//                       rec_c R4[n-1], rec_t int2[n-1] (traversal records)
+//                       rec_c R4[n-1], rec_t int2[n-1] (traversal records),
+//                       bounds float4[n-1] (FP64: of the opening tests)
+//   piece, pieces       what climbs in the tree's second launch (tree.cuh)
 //   bbox, quant         the bounding box and Morton quantisation, computed by
 //                       the displacement of the previous iteration
-//   packed, exact_part  R4[n], R2[rows n]  (exact repulsion only)
+//   packed, exact_part  ExactRec[n], R2[rows n]  (exact repulsion only)
 //   st, status          FP64 speed state, status words
 #pragma once
 

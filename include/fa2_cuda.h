@@ -83,7 +83,8 @@ int fa2cu_layout_traversal_counts(fa2cu_layout *L, double counts[2]);
  * them up in the same order (identical forces), walk 5 in another (forces
  * equal to ~1e-7 in single precision):
  *   "walk"         Barnes-Hut walk: 1 one independent walk per thread
- *                  (default in double precision), 0 warp-synchronous (lanes
+ *                  (default in double precision, where the warp evaluates
+ *                  the lanes' terms together), 0 warp-synchronous (lanes
  *                  walk together, keeping their own decisions), 2 the
  *                  per-thread walk compiled without its register bound, 3 /
  *                  4 two / four Morton neighbours per thread, 5 the regions
