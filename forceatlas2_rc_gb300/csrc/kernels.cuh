@@ -2552,14 +2552,15 @@ k_exact_sum(int n, int rows, const typename RT<R>::R2 *__restrict__ partial,
 
 // Source ranges (rows) of an n-node FP32 all-pairs sum on a GPU of `sms` SMs,
 // of at least 16 sources each: two blocks an SM for small layouts, whose rows
-// the attraction adds up (an iteration in us with 2 / 4 / 8 blocks an SM:
-// 2,000 nodes 19.8 / 22.4 / 22.4; 6,007 30.4 / 32.4 / 37.4; 9,999 48.0 / 48.3 /
-// 50.0), the eight an SM holds for large ones (20,000 133.9 / 126.9 / 124.5;
-// 40,000 516 / 451 / 437; 100,003 - / 2699 / 2591).
+// the attraction adds up (an iteration in us with 1 / 2 / 3 blocks an SM: 3,001
+// nodes 19.3 / 18.6 / 19.5; 4,500 25.5 / 22.1 / 22.6; 9,000 44.5 / 38.7 / 38.8),
+// three for middle ones (12,000 with 2 / 3 / 8: 55.5 / 54.5 / 57.4), the eight
+// an SM holds for large ones (20,000 with 2 / 3 / 8: 132.6 / 127.0 / 122.4;
+// 100,003 with 4 / 8: 2699 / 2591).
 inline int exact_rows(int n, int sms, int ipt)
 {
     const int nb = (n + EXACT_THREADS * ipt - 1) / (EXACT_THREADS * ipt);
-    const int rows = std::min((n < 12000 ? 2 : 8) * sms / nb, n / 16);
+    const int rows = std::min((n < 10000 ? 2 : n < 16000 ? 3 : 8) * sms / nb, n / 16);
     return std::max(1, rows);
 }
 

@@ -50,9 +50,10 @@ inline int device_sms()
 }
 
 // FP32 nodes a thread of the all-pairs kernel: six share a source's loads;
-// with few nodes two, for more threads (4,000 nodes: 23 against 28 us an
-// iteration).
-inline int exact_ipt(int n) { return n < 4096 ? 2 : 6; }
+// with few nodes two, for more threads and fewer rows to add up (an iteration
+// in us with two / six: 4,500 nodes 22.1 / 24.4, 6,007 26.2 / 27.7, 9,000 42.1 /
+// 38.7).
+inline int exact_ipt(int n) { return n < 7000 ? 2 : 6; }
 
 // The all-pairs repulsion of n records. FP32: `rows` rows of partial sums
 // (n entries each; exact_rows) into `partial`, for exact_sum to add up -- or,

@@ -48,3 +48,16 @@ def test_exact_single(gpu, n, adjust):
         L.set_positions(pos)
         assert rel_err(L.forces(pos), want) <= (2e-3 if adjust else 1e-4)
     assert np.isfinite(moved).all()
+
+
+@pytest.mark.parametrize("n", [6999, 7000, 9999, 10000, 15999, 16000])
+def test_exact_single_split(gpu, n):
+    """Where the nodes a thread and the rows of sources change (without radii:
+    among this many nodes some pair is nearer to contact than its float terms
+    are good for)."""
+    _, pos, _, double = _layout(n, "double", False, np.random.default_rng(n))
+    with double as L:
+        want = L.forces(pos)
+    _, _, _, single = _layout(n, "single", False, np.random.default_rng(n))
+    with single as L:
+        assert rel_err(L.forces(pos), want) <= 1e-4
