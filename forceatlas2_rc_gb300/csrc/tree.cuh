@@ -199,7 +199,17 @@ k_tree(int n, int W, int adjust, const uint32_t *__restrict__ order,
     if (i == 0) listed = 0;
     done[i] = made[i] = 0;
     pdl_wait();
+    // the leaf that a thread may have: its node and place are on their way
+    // while the block's edges are found (an iteration of 3,001 nodes 55.3 -> 53.7
+    // us, 10,007 65.0 -> 64.3)
+    const int place = max((int) blockIdx.x * (M - 2 * W) - W, 0) + i;
+    uint32_t node = place < n ? order[place] : 0u;
     for (int j = i; j < M + 4; j += M) code[j] = from + j < n ? key[from + j] : 0u;
+    const bool ok = node < (uint32_t) n; // always, for a valid sort
+    if (!ok) node = 0u;
+    typename RT<R>::R2 p = pos[node];
+    R m = mass[node], sz = R(0);
+    if (adjust) sz = size[node];
     __syncthreads();
     if (i < 64) {
         const int at = tree_edge(blockIdx.x + (i >> 5), n, W, code, from);
@@ -209,21 +219,15 @@ k_tree(int n, int W, int adjust, const uint32_t *__restrict__ order,
     const int s0 = edge[0], s1 = edge[1], cnt = s1 - s0;
     const uint32_t *c0 = code + (s0 - from); // c0[i]: leaf s0 + i
     const signed char *d0 = sep + 1;         // d0[i]: the split after leaf s0 + i; -1 past the ends
-    if (i < cnt) {
-        const uint32_t node = order[s0 + i];
-        const bool ok = node < (uint32_t) n; // always, for a valid sort
-        typename RT<R>::R2 p = mk2<R>(R(0), R(0));
-        R m = R(0), sz = R(0);
-        if (ok) {
-            p = pos[node];
-            m = mass[node];
-            if (adjust) sz = size[node];
-        } else {
+    if (place >= s0 && place < s1) {
+        if (!ok) {
+            p = mk2<R>(R(0), R(0));
+            m = sz = R(0);
             atomicOr(status + ST_ERROR, ERR_BOUNDS);
         }
         const R4 rec = mk4<R>(p.x, p.y, m, sz);
-        leaf[i] = rec;
-        A.psort[s0 + i] = rec;
+        leaf[place - s0] = rec;
+        A.psort[place] = rec;
     }
     for (int j = i - 1; j < cnt + 1; j += M) {
         const int k = s0 + j;
