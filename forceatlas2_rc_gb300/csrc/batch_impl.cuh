@@ -80,18 +80,22 @@ enum { BP_CODES, BP_SORT, BP_TREE, BP_SUMS, BP_REPULSION, BP_ATTRACTION, BP_TOTA
 
 // (block_sort_pairs, the one-block radix sort, is in sort_tree.cuh)
 
-// Sum over the block in a fixed order (per thread, per warp by shuffles, over
-// the warps by thread 0); the result is valid in thread 0.
-template <int W> __device__ double block_sum(double v, double *scratch)
+// Sum over the block in a fixed order (H values per thread, of threads t, t + T,
+// ...; per warp by shuffles, over the warps by thread 0); the result is valid in
+// thread 0.
+template <int W, int H> __device__ double block_sum(const double (&v)[H], double *scratch)
 {
-    v = warp_sum(v);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     __syncthreads();
-    if (lane == 0) scratch[w] = v;
+#pragma unroll
+    for (int h = 0; h < H; h++) {
+        const double x = warp_sum(v[h]);
+        if (lane == 0) scratch[h * W + w] = x;
+    }
     __syncthreads();
     double s = 0.0, c = 0.0;
     if (threadIdx.x == 0)
-        for (int k = 0; k < W; k++) neumaier(s, c, scratch[k]);
+        for (int k = 0; k < W * H; k++) neumaier(s, c, scratch[k]);
     return __dadd_rn(s, c);
 }
 
@@ -99,8 +103,14 @@ template <int W> __device__ double block_sum(double v, double *scratch)
 
 // FP32: two blocks of 512 (four of 256) threads per SM, 64 registers a thread,
 // which the group walk wants (three blocks at 40 registers: 3.01 against 2.85
-// ms an iteration of 1,024 graphs of 50 to 20,000 nodes). FP64 needs more registers: one block of 512 (two
-// of 256).
+// ms an iteration of 1,024 graphs of 50 to 20,000 nodes). FP64 needs more
+// registers: one block of 512 (two of 256).
+// FP32 graphs that would outlast the others (wide_graphs) are taken by blocks
+// of WIDE threads, which have an SM each. They are launched first, and the
+// other blocks when all of them have started (launch_kernel).
+constexpr int WIDE = 1024;
+constexpr int WIDE_MIN = 1024; // nodes, below which such a block has idle threads
+
 template <class R, int T>
 __global__ void __launch_bounds__(T, (sizeof(R) == 8 ? 512 : 1024) / T)
 k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterations,
@@ -109,17 +119,21 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
     typedef typename RT<R>::R2 R2;
     typedef typename RT<R>::R4 R4;
     constexpr int W = T / 32;
+    // the threads that the totals are made for: the same sums whatever T (a
+    // graph's layout does not depend on the batch it is in)
+    constexpr int V = sizeof(R) == 4 ? WIDE : T, H = V / T;
     // the sort's digit counts; in the same space the exact sum's record tile
     // (T records of at most 32 bytes), and the group walk's arrays
     extern __shared__ __align__(16) unsigned char batch_smem[];
     uint32_t(*cnt)[256] = reinterpret_cast<uint32_t(*)[256]>(batch_smem);
     __shared__ uint32_t dbase[256];
-    __shared__ double red[W], red2[W];
+    __shared__ double red[V / 32], red2[V / 32];
     __shared__ R mins[4][W];
     __shared__ double quant[3];
     __shared__ double sh_speed;
     __shared__ int sh_g, sh_stop;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    if (T == WIDE) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     for (;;) {
         if (tid == 0) sh_g = atomicAdd(next, 1);
@@ -392,19 +406,24 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
             // reference's order, as the single-graph path), else per thread
             // and over the block
             const bool serial = serial_totals<R>(n);
-            double ts = 0.0, tt = 0.0;
-            for (int i = tid; i < n; i += T) {
-                const R2 a = f[i], b = fold[i];
-                const R sx = b.x - a.x, sy = b.y - a.y;
-                const R tx = b.x + a.x, ty = b.y + a.y;
-                const R m = mass[i];
-                const R s = m * fsqrt(sx * sx + sy * sy);
-                const R t = R(0.5) * m * fsqrt(tx * tx + ty * ty);
-                sw[i] = s;
-                if (serial) tr[i] = t;
-                if (fixed && fixed[i]) continue;
-                ts = __dadd_rn(ts, (double) s);
-                tt = __dadd_rn(tt, (double) t);
+            double ts[H] = {}, tt[H] = {};
+            for (int i0 = tid; i0 < n; i0 += V) {
+#pragma unroll
+                for (int h = 0; h < H; h++) {
+                    const int i = i0 + h * T;
+                    if (i >= n) break;
+                    const R2 a = f[i], b = fold[i];
+                    const R sx = b.x - a.x, sy = b.y - a.y;
+                    const R tx = b.x + a.x, ty = b.y + a.y;
+                    const R m = mass[i];
+                    const R s = m * fsqrt(sx * sx + sy * sy);
+                    const R t = R(0.5) * m * fsqrt(tx * tx + ty * ty);
+                    sw[i] = s;
+                    if (serial) tr[i] = t;
+                    if (fixed && fixed[i]) continue;
+                    ts[h] = __dadd_rn(ts[h], (double) s);
+                    tt[h] = __dadd_rn(tt[h], (double) t);
+                }
             }
             double tsw = block_sum<W>(ts, red);
             double ttr = block_sum<W>(tt, red2);
@@ -472,6 +491,9 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
             G->efficiency = eff;
         }
     }
+    // (what follows in the stream waits for this grid: it ends after the wide
+    // blocks'; each of those is on an SM already)
+    if (T != WIDE) pdl_wait();
 }
 
 // Dynamic shared memory of k_batch.
@@ -495,7 +517,8 @@ template <class R> struct Batch : BatchBase {
     BatchGraph *graphs = nullptr;
     int *queue = nullptr, *next = nullptr, *status = nullptr;
     std::vector<int> node0, nsize;
-    int blocks = 0;
+    int blocks = 0;                // of `threads`
+    int nwide = 0, wide_blocks = 0; // the first nwide graphs of the queue: blocks of WIDE
     std::map<int, cudaGraphExec_t> execs; // iteration count -> captured launch
 
     ~Batch() override
@@ -565,7 +588,7 @@ template <class R> struct Batch : BatchBase {
         A.rec_t = mem.get<int2>(n1);
         graphs = mem.get<BatchGraph>((size_t) G);
         queue = mem.get<int>((size_t) G);
-        next = mem.get<int>(1);
+        next = mem.get<int>(2); // of the wide blocks, of the others
         status = mem.get<int>(ST_COUNT);
         if (mem.failed) {
             set_cuda_error("could not allocate memory on the device", mem.err);
@@ -621,11 +644,18 @@ template <class R> struct Batch : BatchBase {
         // largest work first: a block that takes a graph lays it out to the end
         std::vector<int> hq(G);
         std::iota(hq.begin(), hq.end(), 0);
-        std::stable_sort(hq.begin(), hq.end(), [&](int a, int b) {
-            const double ca = hg[a].exact ? (double) hg[a].n * hg[a].n : 300.0 * hg[a].n;
-            const double cb = hg[b].exact ? (double) hg[b].n * hg[b].n : 300.0 * hg[b].n;
-            return ca > cb;
-        });
+        auto cost = [&](int g) {
+            return hg[g].exact ? (double) hg[g].n * hg[g].n : 300.0 * hg[g].n;
+        };
+        std::stable_sort(hq.begin(), hq.end(), [&](int a, int b) { return cost(a) > cost(b); });
+        int sms = 0, per_sm = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+        if constexpr (sizeof(R) == 4) {
+            const std::vector<char> wide = wide_graphs(cost, hg.data(), sms);
+            nwide = (int) (std::stable_partition(hq.begin(), hq.end(),
+                                                 [&](int g) { return wide[g]; }) -
+                           hq.begin());
+        }
         int rc = 0;
         auto up = [&](void *dst, const void *src, size_t bytes) {
             if (!rc && bytes)
@@ -646,8 +676,6 @@ template <class R> struct Batch : BatchBase {
             set_cuda_error("could not send the batch to the device", cudaGetLastError());
             return 1;
         }
-        int sms = 0, per_sm = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         auto setup = [&](auto kernel, int th, size_t smem) {
             FA2_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int) smem),
@@ -655,11 +683,40 @@ template <class R> struct Batch : BatchBase {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, th, smem);
             return 0;
         };
+        if constexpr (sizeof(R) == 4) {
+            if (nwide && setup(k_batch<R, WIDE>, WIDE, batch_smem_bytes<R, WIDE>())) return 1;
+            wide_blocks = std::min(nwide, sms * std::max(per_sm, 1));
+        }
         if (threads == 256 ? setup(k_batch<R, 256>, 256, batch_smem_bytes<R, 256>())
                            : setup(k_batch<R, 512>, 512, batch_smem_bytes<R, 512>()))
             return 1;
-        blocks = std::max(1, std::min(G, sms * std::max(per_sm, 1)));
+        blocks = std::min(G - nwide, sms * std::max(per_sm, 1));
         return 0;
+    }
+
+    // The graphs that blocks of WIDE threads lay out: those over the tree whose
+    // work is more than 0.55 of an SM's share of the whole (if these are more
+    // than the SMs: more than the share). A block of 512 on half an SM would
+    // still be at work on them when the others are done.
+    // 10 iterations in ms, blocks of 512 and with wide ones: 1,024 graphs of 50
+    // to 20,000 nodes 29.3 -> 16.0, 300 of 50 to 8,000 10.4 -> 6.2, ten of
+    // 20,000 21.6 -> 15.6, 152 of 3,000 3.17 -> 2.40, eight of 2,100 2.26 ->
+    // 1.84. 300 of 8,000, all of them wide, 12.0 -> 12.8: two waves of barriers
+    // that nothing hides. Exact graphs of 3,000 nodes 4.4 -> 5.2.
+    template <class Cost> std::vector<char> wide_graphs(Cost cost, const BatchGraph *g, int sms)
+    {
+        double share = 0.0;
+        for (int q = 0; q < G; q++) share += cost(q) / std::max(sms, 1);
+        std::vector<char> wide(G);
+        for (double line : {0.55 * share, share}) {
+            int count = 0;
+            for (int q = 0; q < G; q++) {
+                wide[q] = !g[q].exact && g[q].n >= WIDE_MIN && cost(q) > line;
+                count += wide[q];
+            }
+            if (count <= sms) break;
+        }
+        return wide;
     }
 
     static R2 mk2h(double x, double y)
@@ -670,19 +727,31 @@ template <class R> struct Batch : BatchBase {
         return v;
     }
 
+    // The wide blocks, then (a programmatic launch: when every wide block has
+    // started) the others, on what is left of the GPU.
     void launch_kernel(int iterations, const BatchArrays<R> &arrays)
     {
+        if constexpr (sizeof(R) == 4) {
+            if (nwide)
+                k_batch<R, WIDE><<<wide_blocks, WIDE, batch_smem_bytes<R, WIDE>(), s>>>(
+                    nwide, graphs, queue, next, iterations, arrays, npt, status);
+        }
+        if (G == nwide) return;
+        BatchArrays<R> rest = arrays;
+        if (rest.prof) rest.prof += (size_t) wide_blocks * 8;
+        auto go = [&](auto kernel, size_t smem) {
+            launch_k(nwide > 0, kernel, dim3(blocks), dim3(threads), smem, s, G - nwide, graphs,
+                     (const int *) (queue + nwide), next + 1, iterations, rest, npt, status);
+        };
         if (threads == 256)
-            k_batch<R, 256><<<blocks, 256, batch_smem_bytes<R, 256>(), s>>>(
-                G, graphs, queue, next, iterations, arrays, npt, status);
+            go(k_batch<R, 256>, batch_smem_bytes<R, 256>());
         else
-            k_batch<R, 512><<<blocks, 512, batch_smem_bytes<R, 512>(), s>>>(
-                G, graphs, queue, next, iterations, arrays, npt, status);
+            go(k_batch<R, 512>, batch_smem_bytes<R, 512>());
     }
 
     void launch(int iterations)
     {
-        cudaMemsetAsync(next, 0, sizeof(int), s);
+        cudaMemsetAsync(next, 0, 2 * sizeof(int), s);
         launch_kernel(iterations, A);
     }
 
@@ -724,18 +793,18 @@ template <class R> struct Batch : BatchBase {
     {
         cudaSetDevice(device);
         DevMem tmp;
-        unsigned long long *prof = tmp.get<unsigned long long>((size_t) blocks * 8);
+        const size_t count = (size_t) (wide_blocks + blocks) * 8;
+        unsigned long long *prof = tmp.get<unsigned long long>(count);
         if (tmp.failed) {
             set_cuda_error("could not allocate memory on the device", tmp.err);
             return 1;
         }
-        int rc = cudaMemsetAsync(prof, 0, (size_t) blocks * 8 * sizeof(unsigned long long), s) !=
-                 cudaSuccess;
+        int rc = cudaMemsetAsync(prof, 0, count * sizeof(unsigned long long), s) != cudaSuccess;
         BatchArrays<R> P = A;
         P.prof = prof;
-        if (!rc) rc = cudaMemsetAsync(next, 0, sizeof(int), s) != cudaSuccess;
+        if (!rc) rc = cudaMemsetAsync(next, 0, 2 * sizeof(int), s) != cudaSuccess;
         if (!rc) launch_kernel(iterations, P);
-        std::vector<unsigned long long> h((size_t) blocks * 8);
+        std::vector<unsigned long long> h(count);
         if (!rc)
             rc = cudaMemcpyAsync(h.data(), prof, h.size() * sizeof(unsigned long long),
                                  cudaMemcpyDeviceToHost, s) != cudaSuccess;
@@ -746,8 +815,7 @@ template <class R> struct Batch : BatchBase {
             return 1;
         }
         for (int k = 0; k < 8; k++) out[k] = 0.0;
-        for (size_t b = 0; b < (size_t) blocks; b++)
-            for (int k = 0; k < 8; k++) out[k] += (double) h[b * 8 + k];
+        for (size_t b = 0; b < count; b++) out[b % 8] += (double) h[b];
         return 0;
     }
 
