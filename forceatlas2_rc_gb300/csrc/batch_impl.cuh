@@ -99,6 +99,31 @@ template <int W, int H> __device__ double block_sum(const double (&v)[H], double
     return __dadd_rn(s, c);
 }
 
+// Two sums over the block of V threads' values each (H a thread), added in pairs:
+// by warp, then the V / 32 warps' sums by a warp each. Into a[0] and b[0].
+template <int W, int H>
+__device__ void block_sums(const double (&x)[H], const double (&y)[H], double *a, double *b)
+{
+    static_assert(W * H == 32 && W >= 2, "a lane per warp's sum");
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int h = 0; h < H; h++) {
+        const double u = warp_sum(x[h]), v = warp_sum(y[h]);
+        if (lane == 0) {
+            a[h * W + w] = u;
+            b[h * W + w] = v;
+        }
+    }
+    __syncthreads();
+    if (w < 2) {
+        double *v = w == 0 ? a : b;
+        const double sum = warp_sum(v[lane]);
+        __syncwarp();
+        if (lane == 0) v[0] = sum;
+    }
+    __syncthreads();
+}
+
 // ---- the persistent kernel -----------------------------------------------------
 
 // FP32: two blocks of 512 (four of 256) threads per SM, 64 registers a thread,
@@ -129,7 +154,8 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
     __shared__ uint32_t dbase[256];
     __shared__ double red[V / 32], red2[V / 32];
     __shared__ R mins[4][W];
-    __shared__ double quant[3];
+    __shared__ __align__(16) double quant[6]; // (as k_bbox makes it)
+    __shared__ SpeedTerms terms;
     __shared__ double sh_speed;
     __shared__ int sh_g, sh_stop;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -169,6 +195,7 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
         if (tid == 0) {
             sh_speed = G->speed;
             sh_stop = 0;
+            terms = speed_terms(n);
         }
         double speed = G->speed, eff = G->efficiency;
 
@@ -305,23 +332,12 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
                         mxx = cl_max(mxx, mins[2][k]);
                         mxy = cl_max(mxy, mins[3][k]);
                     }
-                    const double wd = __dsub_rn((double) mxx, (double) mnx);
-                    const double hd = __dsub_rn((double) mxy, (double) mny);
-                    const double ext = cl_max(wd, hd);
-                    quant[0] = (double) mnx;
-                    quant[1] = (double) mny;
-                    quant[2] = ext > 0.0 ? __ddiv_rn(65535.0, ext) : 0.0;
+                    quant_make<R>(mnx, mny, mxx, mxy, quant);
                 }
                 __syncthreads();
+                const MortonQuant<R> Q(quant);
                 for (int i = tid; i < n; i += T) {
-                    const R2 p = pos[i];
-                    const double fx = cl_min(
-                        cl_max(__dmul_rn(__dsub_rn((double) p.x, quant[0]), quant[2]), 0.0),
-                        65535.0);
-                    const double fy = cl_min(
-                        cl_max(__dmul_rn(__dsub_rn((double) p.y, quant[1]), quant[2]), 0.0),
-                        65535.0);
-                    key[i] = spread16((uint32_t) fx) | (spread16((uint32_t) fy) << 1);
+                    key[i] = Q.key(pos[i]);
                     idx[i] = (uint32_t) i;
                 }
                 __syncthreads();
@@ -425,8 +441,17 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
                     tt[h] = __dadd_rn(tt[h], (double) t);
                 }
             }
-            double tsw = block_sum<W>(ts, red);
-            double ttr = block_sum<W>(tt, red2);
+            double tsw, ttr;
+            if constexpr (sizeof(R) == 4) {
+                // both at once, by pairs to the end (a serial sum over the
+                // warps, compensated, took 100 dependent FP64 operations)
+                block_sums<W>(ts, tt, red, red2);
+                tsw = red[0];
+                ttr = red2[0];
+            } else {
+                tsw = block_sum<W>(ts, red);
+                ttr = block_sum<W>(tt, red2);
+            }
             if (serial) {
                 __syncthreads(); // sw / tr written by every thread
                 if (tid < 64) { // a warp each
@@ -449,9 +474,8 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
                     SpeedState s0;
                     s0.speed = speed;
                     s0.efficiency = eff;
-                    s0.n = n;
                     s0.jitter_tolerance = G->jitter;
-                    update_speed_dev(&s0, tsw, ttr);
+                    update_speed(&s0, terms, tsw, ttr);
                     speed = s0.speed;
                     eff = s0.efficiency;
                     sh_speed = speed;

@@ -154,6 +154,25 @@ template <class T> __device__ __forceinline__ T warp_sum(T v)
     return v;
 }
 
+// The Morton quantisation of a bounding box, in double (pipeline.cl:122-124);
+// for the float quantisation (MortonQuant) also the scale as a float-float pair
+// (hi, lo) and the minima as floats, in slots 4 and 5, 16-byte aligned.
+template <class R>
+__device__ __forceinline__ void quant_make(R minx, R miny, R maxx, R maxy, double *quant)
+{
+    const double w = __dsub_rn((double) maxx, (double) minx);
+    const double h = __dsub_rn((double) maxy, (double) miny);
+    const double extent = cl_max(w, h);
+    quant[0] = (double) minx;
+    quant[1] = (double) miny;
+    quant[2] = extent > 0.0 ? __ddiv_rn(65535.0, extent) : 0.0;
+    float *qf = reinterpret_cast<float *>(quant + 4);
+    qf[0] = (float) quant[2];
+    qf[1] = (float) (quant[2] - (double) qf[0]);
+    qf[2] = minx;
+    qf[3] = miny;
+}
+
 // ---- 1. bounding box (pipeline.cl:61-99) ----------------------------------
 // Block partial minima / maxima, then the last block to finish reduces the
 // partials: min and max are exact, so the result does not depend on order.
@@ -234,20 +253,7 @@ __device__ __forceinline__ void bbox_finish(R mnx, R mny, R mxx, R mxy, R *parti
         bbox[1] = b;
         bbox[2] = c;
         bbox[3] = d;
-        // the Morton quantisation of pipeline.cl:122-124, in double
-        const double w = __dsub_rn((double) c, (double) a), h = __dsub_rn((double) d, (double) b);
-        const double extent = cl_max(w, h);
-        quant[0] = (double) a;
-        quant[1] = (double) b;
-        quant[2] = extent > 0.0 ? __ddiv_rn(65535.0, extent) : 0.0;
-        // for the float quantisation of k_morton: the scale as a float-float
-        // pair (hi, lo) and the minima as floats, 16-byte aligned in slots
-        // 4 and 5
-        float *qf = reinterpret_cast<float *>(quant + 4);
-        qf[0] = (float) quant[2];
-        qf[1] = (float) (quant[2] - (double) qf[0]);
-        qf[2] = a;
-        qf[3] = b;
+        quant_make<R>(a, b, c, d, quant);
         *ticket = 0u;
     }
 }
