@@ -124,6 +124,143 @@ __device__ void block_sums(const double (&x)[H], const double (&y)[H], double *a
     __syncthreads();
 }
 
+// The all-pairs repulsion of an FP32 graph of at most T nodes by its block of T
+// threads, into f: two nodes a thread, packed (the terms of k_exact), the sources
+// in shared memory and split over the threads, the parts' sums added in order.
+//
+// Bound by latency: barriers and a chain of n / parts sources. With a thread a
+// node (block_exact_tiles) a graph left most threads idle; 10 iterations in ms:
+// eight graphs of 60 nodes 0.226 -> 0.099, of 500 0.357 -> 0.262; 2,000 of 100
+// nodes 1.82 -> 0.84, of 300 2.47 -> 1.31. Above T nodes these are faster (3,000
+// nodes 4.4 against 5.7, 1,100 1.27 against 1.29: as many MUFU operations, and a
+// longer record to load for each pair of nodes).
+constexpr int BATCH_PARTS = 16; // at most
+
+template <int T> constexpr size_t block_exact_smem()
+{
+    return T * (sizeof(ExactF32) + 2 * sizeof(float2));
+}
+
+template <bool ADJUST, int T>
+__device__ __noinline__ void block_exact(int n, float scaling, const float2 *pos,
+                                         const float *mass, const float *size, float2 *f,
+                                         unsigned char *smem)
+{
+    ExactF32 *const rec = reinterpret_cast<ExactF32 *>(smem); // T
+    float2 *const part = reinterpret_cast<float2 *>(rec + T); // 2 T
+    const int tid = threadIdx.x, half = (n + 1) / 2;
+    const int parts = min(BATCH_PARTS, T / half); // (2 at least: half <= T / 2)
+    const int q = tid / half, slot = tid - q * half;
+    if (tid < n) exact_fill(rec + tid, pos[tid], mass[tid], ADJUST ? size[tid] : 0.0f);
+    __syncthreads();
+    if (q < parts) {
+        const ExactF32 a = rec[slot], b = rec[min(slot + half, n - 1)];
+        GroupNode me;
+        me.x = f2_make(-a.nx[0], -b.nx[0]);
+        me.y = f2_make(-a.ny[0], -b.ny[0]);
+        const float sa = a.r[0], sb = b.r[0];
+        f2 ax = 0, ay = 0;
+        const int seg = (n + parts - 1) / parts;
+        const int from = min(n, q * seg), to = min(n, from + seg);
+        unsigned at = smem_addr(rec + from);
+#pragma unroll 4
+        for (int j = from; j < to; j++, at += (unsigned) sizeof(ExactF32)) {
+            f2 nx, ny, mm, r = 0;
+            lds_2<0>(at, nx, ny);
+            if (ADJUST)
+                lds_2<16>(at, mm, r);
+            else
+                mm = lds_1<16>(at);
+            exact_term<ADJUST>(me, sa, sb, nx, ny, mm, r, ax, ay);
+        }
+        float xa, xb, ya, yb;
+        f2_split(ax, xa, xb);
+        f2_split(ay, ya, yb);
+        part[q * n + slot] = make_float2(xa, ya);
+        if (slot + half < n) part[q * n + slot + half] = make_float2(xb, yb);
+    }
+    __syncthreads();
+    if (tid < n) {
+        float2 v = part[tid];
+        for (int r = 1; r < parts; r++) {
+            const float2 o = part[r * n + tid];
+            v.x += o.x;
+            v.y += o.y;
+        }
+        const float m = scaling * rec[tid].m[0];
+        f[tid] = make_float2(v.x * m, v.y * m);
+    }
+}
+
+// The same of a larger graph, or in FP64: every node's sum by a thread, over
+// tiles of T records staged in shared memory, in node order. two: the tile shape
+// (autotuned), two nodes per thread (i and i + T), each tile record feeding two
+// independent sums, or one; every node sums j ascending either way. (Inlined and
+// unrolled: eight FP32 graphs of 3,000 nodes, 10 iterations, 4.6 ms; a function
+// of its own 5.8, unrolled by four 4.7, not at all 5.4.)
+template <class R, bool ADJUST, int T>
+__device__ __forceinline__ void block_exact_tiles(int n, bool two, R scaling,
+                                               const typename RT<R>::R2 *pos, const R *mass,
+                                               const R *size, typename RT<R>::R4 *psort,
+                                               typename RT<R>::R2 *f, unsigned char *smem)
+{
+    typedef typename RT<R>::R2 R2;
+    typedef typename RT<R>::R4 R4;
+    const int tid = threadIdx.x;
+    R4 *const tile = reinterpret_cast<R4 *>(smem);
+    for (int i = tid; i < n; i += T) {
+        const R2 p = pos[i];
+        psort[i] = mk4<R>(p.x, p.y, mass[i], ADJUST ? size[i] : R(0));
+    }
+    for (int i0 = 0; i0 < n; i0 += two ? 2 * T : T) {
+        const int ia = i0 + tid, ib = two ? ia + T : n;
+        const R4 zero = mk4<R>(R(0), R(0), R(0), R(0));
+        const R4 ma = ia < n ? psort[ia] : zero, mb = ib < n ? psort[ib] : zero;
+        R axa = R(0), aya = R(0), axb = R(0), ayb = R(0);
+        for (int j0 = 0; j0 < n; j0 += T) {
+            __syncthreads();
+            if (j0 + tid < n) tile[tid] = psort[j0 + tid];
+            __syncthreads();
+            const int m = min(T, n - j0);
+            // one source on a node (FP32 without radii: d2 carries 1e-30, as in
+            // k_exact, and scaling * m_i comes once, at the end)
+            auto add = [&](const R4 &me, const R4 &q, R &ax, R &ay) {
+                const R xd = me.x - q.x, yd = me.y - q.y;
+                if constexpr (sizeof(R) == 4 && !ADJUST) {
+                    const float g = q.z * __fdividef(1.0f, fmaf(xd, xd, fmaf(yd, yd, 1e-30f)));
+                    ax = fmaf(xd, g, ax);
+                    ay = fmaf(yd, g, ay);
+                } else {
+                    const R g = rep_factor<R, ADJUST>(xd * xd + yd * yd, me.z * q.z,
+                                                      ADJUST ? me.w + q.w : R(0), scaling);
+                    ax += xd * g;
+                    ay += yd * g;
+                }
+            };
+            if (two) {
+#pragma unroll 16
+                for (int jj = 0; jj < m; jj++) {
+                    const R4 q = tile[jj];
+                    add(ma, q, axa, aya);
+                    add(mb, q, axb, ayb);
+                }
+            } else {
+#pragma unroll 8
+                for (int jj = 0; jj < m; jj++) add(ma, tile[jj], axa, aya);
+            }
+        }
+        if (sizeof(R) == 4 && !ADJUST) {
+            const R sa = scaling * ma.z, sb = scaling * mb.z;
+            axa *= sa;
+            aya *= sa;
+            axb *= sb;
+            ayb *= sb;
+        }
+        if (ia < n) f[ia] = mk2<R>(axa, aya);
+        if (ib < n) f[ib] = mk2<R>(axb, ayb);
+    }
+}
+
 // ---- the persistent kernel -----------------------------------------------------
 
 // FP32: two blocks of 512 (four of 256) threads per SM, 64 registers a thread,
@@ -213,95 +350,21 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
             phase(BP_MOVE);
             if (sh_stop) break;
             if (exact || n < 2) {
-                // records in original order; the all-pairs sum per node over
-                // tiles of T records staged in shared memory (in node order)
-                for (int i = tid; i < n; i += T) {
-                    const R2 p = pos[i];
-                    psort[i] = mk4<R>(p.x, p.y, mass[i], adjust ? size[i] : R(0));
-                }
-                R4 *tile = reinterpret_cast<R4 *>(&cnt[0][0]);
-                // the tile shape (autotuned): npt = 2 nodes per thread (i
-                // and i + T), each tile record feeding two independent sums,
-                // or 1; every node sums j ascending either way
                 const bool two = npt == 2 && n > T;
-                for (int i0 = 0; i0 < n; i0 += two ? 2 * T : T) {
-                    const int ia = i0 + tid, ib = two ? ia + T : n;
-                    const R4 zero = mk4<R>(R(0), R(0), R(0), R(0));
-                    const R4 ma = ia < n ? psort[ia] : zero, mb = ib < n ? psort[ib] : zero;
-                    R axa = R(0), aya = R(0), axb = R(0), ayb = R(0);
-                    const float smia = (float) scaling * (float) ma.z;
-                    const float smib = (float) scaling * (float) mb.z;
-                    for (int j0 = 0; j0 < n; j0 += T) {
-                        __syncthreads();
-                        if (j0 + tid < n) tile[tid] = psort[j0 + tid];
-                        __syncthreads();
-                        const int m = min(T, n - j0);
-                        if (sizeof(R) == 4 && !adjust) {
-                            // d2 carries 1e-30 (as k_exact): a coincident
-                            // pair (xd = yd = 0) has a finite factor, so it
-                            // adds 0, the reference's factor for d2 = 0
-                            if (!two) { // one node per thread
-#pragma unroll 4
-                                for (int jj = 0; jj < m; jj++) {
-                                    const R4 q = tile[jj];
-                                    const float xda = (float) ma.x - (float) q.x;
-                                    const float yda = (float) ma.y - (float) q.y;
-                                    const float d2a = fmaf(xda, xda, fmaf(yda, yda, 1e-30f));
-                                    const float ga = (float) q.z * __fdividef(1.0f, d2a);
-                                    axa = (R) fmaf(xda, ga, (float) axa);
-                                    aya = (R) fmaf(yda, ga, (float) aya);
-                                }
-                            } else {
-#pragma unroll 4
-                                for (int jj = 0; jj < m; jj++) {
-                                    const R4 q = tile[jj];
-                                    const float xda = (float) ma.x - (float) q.x;
-                                    const float yda = (float) ma.y - (float) q.y;
-                                    const float xdb = (float) mb.x - (float) q.x;
-                                    const float ydb = (float) mb.y - (float) q.y;
-                                    const float d2a = fmaf(xda, xda, fmaf(yda, yda, 1e-30f));
-                                    const float d2b = fmaf(xdb, xdb, fmaf(ydb, ydb, 1e-30f));
-                                    const float ga = (float) q.z * __fdividef(1.0f, d2a);
-                                    const float gb = (float) q.z * __fdividef(1.0f, d2b);
-                                    axa = (R) fmaf(xda, ga, (float) axa);
-                                    aya = (R) fmaf(yda, ga, (float) aya);
-                                    axb = (R) fmaf(xdb, gb, (float) axb);
-                                    ayb = (R) fmaf(ydb, gb, (float) ayb);
-                                }
-                            }
-                        } else {
-                            for (int jj = 0; jj < m; jj++) {
-                                const R4 q = tile[jj];
-                                const R xda = ma.x - q.x, yda = ma.y - q.y;
-                                const R xdb = mb.x - q.x, ydb = mb.y - q.y;
-                                R ga, gb;
-                                if (adjust) {
-                                    ga = rep_factor<R, true>(xda * xda + yda * yda, ma.z * q.z,
-                                                             ma.w + q.w, scaling);
-                                    gb = rep_factor<R, true>(xdb * xdb + ydb * ydb, mb.z * q.z,
-                                                             mb.w + q.w, scaling);
-                                } else {
-                                    ga = rep_factor<R, false>(xda * xda + yda * yda, ma.z * q.z,
-                                                              R(0), scaling);
-                                    gb = rep_factor<R, false>(xdb * xdb + ydb * ydb, mb.z * q.z,
-                                                              R(0), scaling);
-                                }
-                                axa += xda * ga;
-                                aya += yda * ga;
-                                axb += xdb * gb;
-                                ayb += ydb * gb;
-                            }
-                        }
-                    }
-                    if (sizeof(R) == 4 && !adjust) { // scaling * m_i, once
-                        axa = (R) ((float) axa * smia);
-                        aya = (R) ((float) aya * smia);
-                        axb = (R) ((float) axb * smib);
-                        ayb = (R) ((float) ayb * smib);
-                    }
-                    if (ia < n) f[ia] = mk2<R>(axa, aya);
-                    if (ib < n) f[ib] = mk2<R>(axb, ayb);
+                bool small = false;
+                if constexpr (sizeof(R) == 4) {
+                    small = n <= T;
+                    if (small && adjust)
+                        block_exact<true, T>(n, scaling, pos, mass, size, f, batch_smem);
+                    else if (small)
+                        block_exact<false, T>(n, scaling, pos, mass, size, f, batch_smem);
                 }
+                if (!small && adjust)
+                    block_exact_tiles<R, true, T>(n, two, scaling, pos, mass, size, psort, f,
+                                                  batch_smem);
+                else if (!small)
+                    block_exact_tiles<R, false, T>(n, two, scaling, pos, mass, size, psort, f,
+                                                   batch_smem);
             } else {
                 // bounding box and the Morton quantisation
                 R mnx = pos[0].x, mxx = mnx, mny = pos[0].y, mxy = mny;
@@ -526,6 +589,7 @@ template <class R, int T> constexpr size_t batch_smem_bytes()
     const size_t sort = (size_t) (T / 32) * 256 * sizeof(uint32_t);
     const size_t walk =
         sizeof(R) == 4 ? sizeof(GroupTopShared) + (T / 32) * sizeof(GroupWalkShared) : 0;
+    static_assert(sizeof(R) == 8 || walk >= block_exact_smem<T>(), "the exact sum's arrays fit");
     return sort > walk ? sort : walk;
 }
 
