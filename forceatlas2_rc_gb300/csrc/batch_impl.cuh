@@ -538,7 +538,8 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
                     s0.speed = speed;
                     s0.efficiency = eff;
                     s0.jitter_tolerance = G->jitter;
-                    update_speed(&s0, terms, tsw, ttr);
+                    s0.terms = terms;
+                    update_speed(&s0, tsw, ttr);
                     speed = s0.speed;
                     eff = s0.efficiency;
                     sh_speed = speed;

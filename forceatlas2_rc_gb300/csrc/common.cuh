@@ -122,11 +122,24 @@ enum {
 
 // Speed-controller state on the device, in double (reference
 // src/forceatlas2.c:445-485 runs it on the host; here it never leaves HBM).
+// What the speed update needs of the number of nodes, made once a layout (the
+// two square roots took the totals' last thread about 2 us an iteration).
+struct SpeedTerms {
+    double est, min_jt, n2;
+};
+inline __host__ __device__ SpeedTerms speed_terms(int n)
+{
+    SpeedTerms t;
+    t.est = 0.05 * sqrt((double) n);
+    t.min_jt = sqrt(t.est);
+    t.n2 = (double) n * (double) n;
+    return t;
+}
 struct SpeedState {
     double speed, efficiency;
     double total_swinging, total_traction;
     double jitter_tolerance;
-    int n, pad;
+    SpeedTerms terms;
 };
 
 // ---- precision traits -----------------------------------------------------

@@ -1726,21 +1726,9 @@ __device__ __forceinline__ void neumaier(double &s, double &c, double v)
     s = t;
 }
 
-// What the speed update needs of the number of nodes.
-struct SpeedTerms {
-    double est, min_jt, n2;
-};
-__device__ inline SpeedTerms speed_terms(int n)
+__device__ inline void update_speed(SpeedState *st, double tsw, double ttr)
 {
-    SpeedTerms t;
-    t.est = __dmul_rn(0.05, sqrt((double) n));
-    t.min_jt = sqrt(t.est);
-    t.n2 = __dmul_rn((double) n, (double) n);
-    return t;
-}
-
-__device__ inline void update_speed(SpeedState *st, const SpeedTerms &T, double tsw, double ttr)
-{
+    const SpeedTerms T = st->terms;
     double speed = st->speed, eff = st->efficiency;
     st->total_swinging = tsw;
     st->total_traction = ttr;
@@ -1766,11 +1754,6 @@ __device__ inline void update_speed(SpeedState *st, const SpeedTerms &T, double 
     st->speed = speed;
     st->efficiency = eff;
 }
-__device__ inline void update_speed_dev(SpeedState *st, double tsw, double ttr)
-{
-    update_speed(st, speed_terms(st->n), tsw, ttr);
-}
-
 // In the FP64 path, up to this many nodes the totals are summed serially in
 // node order, the reference's order (src/forceatlas2.c:770-775): the speed,
 // hence the whole trajectory, is then the reference's bit for bit. Beyond,
@@ -1979,6 +1962,8 @@ __device__ __forceinline__ void swing_finish(SwingAcc<R> acc, int n, const uint8
     __syncthreads();
     if (!last) return;
     __threadfence();
+    SpeedState s; // (on its way beside the partial sums)
+    if (threadIdx.x == 0) s = *st;
     double tsw = 0.0, ttr = 0.0;
     if (serial_totals<R>(n)) {
         // the block stages the nodes' values in shared memory (dynamic, 2n
@@ -2065,7 +2050,8 @@ __device__ __forceinline__ void swing_finish(SwingAcc<R> acc, int n, const uint8
             st->total_swinging = tsw;
             st->total_traction = ttr;
         } else {
-            update_speed_dev(st, tsw, ttr);
+            update_speed(&s, tsw, ttr);
+            *st = s;
         }
     }
 }

@@ -557,7 +557,7 @@ template <class R> struct Layout : LayoutBase {
         h.speed = 1.0;
         h.efficiency = 1.0;
         h.jitter_tolerance = p->jitter_tolerance;
-        h.n = n;
+        h.terms = speed_terms(n);
         FA2_TRY(cudaMemcpyAsync(st, &h, sizeof(h), cudaMemcpyHostToDevice, s), "cudaMemcpy", 1);
         FA2_TRY(cudaStreamSynchronize(s), "could not prepare the layout", 1);
         if (n <= SE_MAX) pick_small(n <= 200 ? 1 : CS_MAX_BLOCKS);

@@ -88,7 +88,6 @@ k_small_exact(int n, int m, int iterations, float scaling, float gravity, int st
     const int j0 = min(n, q * seg), j1 = q < parts ? min(n, j0 + seg) : j0;
     __syncthreads();
     cluster_barrier(); // every block has started, and read the speed and status
-    const SpeedTerms terms = speed_terms(speed.n);
     float2 f = make_float2(0.0f, 0.0f);
     for (int it = 0; it < iterations; it++) {
         // repulsion: the thread's part (the terms of k_exact)
@@ -172,7 +171,7 @@ k_small_exact(int n, int m, int iterations, float scaling, float gravity, int st
                     stop = 1;
                     if (rank == 0) atomicOr(status + ST_ERROR, ERR_NAN);
                 } else {
-                    update_speed(&speed, terms, a, b);
+                    update_speed(&speed, a, b);
                 }
             }
         }
