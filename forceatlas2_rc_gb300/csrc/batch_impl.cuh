@@ -100,15 +100,21 @@ template <int W, int H> __device__ double block_sum(const double (&v)[H], double
 }
 
 // Two sums over the block of V threads' values each (H a thread), added in pairs:
-// by warp, then the V / 32 warps' sums by a warp each. Into a[0] and b[0].
+// by warp, then the V / 32 warps' sums by a warp each. Into a[0] and b[0]. Warps
+// that hold none of the n values have 0 and add nothing up (an FP64 instruction
+// of a warp takes the SM 16 cycles).
 template <int W, int H>
-__device__ void block_sums(const double (&x)[H], const double (&y)[H], double *a, double *b)
+__device__ void block_sums(int n, const double (&x)[H], const double (&y)[H], double *a, double *b)
 {
     static_assert(W * H == 32 && W >= 2, "a lane per warp's sum");
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int h = 0; h < H; h++) {
-        const double u = warp_sum(x[h]), v = warp_sum(y[h]);
+        double u = 0.0, v = 0.0;
+        if (32 * (h * W + w) < n) {
+            u = warp_sum(x[h]);
+            v = warp_sum(y[h]);
+        }
         if (lane == 0) {
             a[h * W + w] = u;
             b[h * W + w] = v;
@@ -508,7 +514,7 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
             if constexpr (sizeof(R) == 4) {
                 // both at once, by pairs to the end (a serial sum over the
                 // warps, compensated, took 100 dependent FP64 operations)
-                block_sums<W>(ts, tt, red, red2);
+                block_sums<W>(n, ts, tt, red, red2);
                 tsw = red[0];
                 ttr = red2[0];
             } else {
