@@ -191,9 +191,11 @@ typedef struct fa2cu_batch fa2cu_batch;
  * positions (x then y). Device and precision are those of graphs[0].
  * Graphs with fewer than exact_below nodes use the exact repulsion, the others
  * Barnes-Hut over their own Morton/Karras tree; threads is the block size
- * (256 or 512); nodes_per_thread (1 or 2) the tile shape of the exact sum
+ * (256 or 512; single-precision graphs over the tree that would outlast the
+ * others have 1024); nodes_per_thread (1 or 2) the tile shape of the exact sum
  * (each thread sums that many nodes against the block's tile of `threads`
- * records in shared memory). exact_below < 0, threads == 0 or
+ * records in shared memory; no difference to single-precision graphs of at most
+ * `threads` nodes). exact_below < 0, threads == 0 or
  * nodes_per_thread == 0: the values measured by fa2cu_batch_tune on this
  * device. A graph's result does not depend on the other graphs of the batch
  * (nor on the tile shape). NULL on error. */
