@@ -8,6 +8,7 @@
 // mass) use the explicit round-to-nearest intrinsics, which are never fused.
 #pragma once
 
+#include "cluster_exchange.h"
 #include "common.cuh"
 #include "karras.cuh"
 #include "sort_tree.cuh"
@@ -461,11 +462,18 @@ k_codes_sort(int n, int m, const typename RT<R>::R2 *__restrict__ pos,
 {
     constexpr int WARPS = T / 32, PARTS = T / 256; // threads a digit, eight warps each
     extern __shared__ __align__(16) uint2 cs_pairs[];
-    // bytes of the counts, and of the pairs, that arrive in a pass: one phase
-    // of each a pass. A block sends a pass's counts when all its pairs of the
-    // pass before have come, and its pairs when all counts have: nobody
-    // writes what another still reads, nor into a phase not yet begun.
-    __shared__ uint64_t bar_counts, bar_pairs;
+    // bytes of the counts, and of the pairs, that arrive in a pass: a phase of
+    // bar_pairs a pass, of bar_counts every other pass (cs_count_bar).
+    // Counts: a block X sends those of pass p + 1 when it holds those of pass p
+    // of every block Y (its pairs may all be its own: it need not have heard
+    // from anyone since). Y sent them after its phase and its reads of the
+    // counts of p - 1, so the barrier and the half of `table` that p + 1 takes
+    // are free at Y, while the counts of p that others send to Y may still be
+    // under way.
+    // Pairs: X sends those of pass p when it holds the counts of p of every Y,
+    // which Y sent after its phase of the pairs of p - 1 and its last reads of
+    // the array that the pairs of p go to.
+    __shared__ uint64_t bar_counts[CS_COUNT_BARS], bar_pairs;
     __shared__ uint32_t wh[WARPS][256];              // a warp's counts, then their prefix
     __shared__ uint32_t table[2][CS_MAX_BLOCKS][256];   // the blocks' counts, by pass parity
     __shared__ uint32_t lbase[256], gbase[256];
@@ -480,7 +488,7 @@ k_codes_sort(int n, int m, const typename RT<R>::R2 *__restrict__ pos,
     const int rounds = (m + T - 1) / T; // <= ITEMS
     const int first = w * rounds * 32;
     if (threadIdx.x == 0) {
-        mbar_init(&bar_counts, 1);
+        for (int b = 0; b < CS_COUNT_BARS; b++) mbar_init(&bar_counts[b], 1);
         mbar_init(&bar_pairs, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -504,8 +512,9 @@ k_codes_sort(int n, int m, const typename RT<R>::R2 *__restrict__ pos,
     cluster_barrier();
     for (int pass = 0; pass < 4; pass++) {
         const int shift = 8 * pass;
+        uint64_t *const bar_pass = &bar_counts[cs_count_bar(pass)];
         if (threadIdx.x == 0) {
-            mbar_expect(&bar_counts, blocks * 256u * (unsigned) sizeof(uint32_t));
+            mbar_expect(bar_pass, blocks * 256u * (unsigned) sizeof(uint32_t));
             if (pass < 3) mbar_expect(&bar_pairs, (unsigned) cnt * (unsigned) sizeof(uint2));
         }
 #pragma unroll
@@ -558,11 +567,11 @@ k_codes_sort(int n, int m, const typename RT<R>::R2 *__restrict__ pos,
             }
             const uint32_t all = __shfl_sync(0xffffffffu, incl, PARTS - 1, PARTS);
             const uint32_t mine = smem_addr(&table[pass & 1][rank][d]);
-            const uint32_t bar = smem_addr(&bar_counts);
+            const uint32_t bar = smem_addr(bar_pass);
             for (unsigned b = part; b < blocks; b += PARTS)
                 cluster_store(cluster_addr(mine, b), all, cluster_addr(bar, b));
         }
-        late |= !mbar_wait(&bar_counts, pass & 1, 1000000000ull);
+        late |= !mbar_wait(bar_pass, cs_count_parity(pass), 1000000000ull);
         // global places: the digits in order, the blocks in order in a digit
         uint32_t total = 0, prev = 0, own = 0, gincl = 0, lincl = 0;
         if (threadIdx.x < 256) {
