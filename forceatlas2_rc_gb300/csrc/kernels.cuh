@@ -1775,16 +1775,16 @@ template <class R> __host__ __device__ constexpr bool serial_totals(int n)
     return sizeof(R) == 8 && n <= SERIAL_TOTALS_MAX;
 }
 
-// v(0) + v(1) + ... + v(n - 1), none negative, added to 0 in that order and
-// rounded after each addition: the bits of the serial sum, by a whole warp
-// (every lane gets it).
+// v(0) + v(1) + ... + v(n - 1), added to 0 in that order and rounded after each
+// addition: the bits of the serial sum, by a whole warp (every lane gets it).
 //
 // While the sum s stays in one binade its roundings are to one spacing u, and s
 // is a multiple of u: fl(s + v) = s + (v rounded to a multiple of u), unless v
 // lies half-way between two. So 128 values are rounded alone and their prefix
 // sums taken, in integers that count the u's. The first value that is half-way,
-// that takes s out of the binade, or that is half of the binade's lower end or
-// more is added by an addition.
+// that takes s out of the binade, that is half of the binade's lower end or more
+// (or no finite number), or that has a sign bit (the GPU's own NaN has) is added
+// by an addition.
 //
 // Why: a dependent FP64 addition takes 64 cycles. The attraction with the
 // totals of 1,500 nodes (both sums, and their staging): 88 us serially, 40 with
@@ -1796,8 +1796,8 @@ template <class F> __device__ inline double ordered_sum(int n, F v)
     double s = 0.0;
     for (int i = 0; i < n;) {
         const long long bits = __double_as_longlong(s);
-        const long long E = bits >> 52; // (s >= 0, or not a number)
-        if (E < 64 || E > 2000) {       // tiny, or no finite sum
+        const long long E = bits >> 52; // (below 0 with a sign bit)
+        if (E < 64 || E > 2000) {       // negative, tiny, or no finite sum
             s = __dadd_rn(s, v(i));
             i++;
             continue;
@@ -1816,7 +1816,7 @@ template <class F> __device__ inline double ordered_sum(int n, F v)
             const int d = (int) min(E - e, 62LL);
             const long long half = 1LL << (d > 0 ? d - 1 : 0), rest = m & (2 * half - 1);
             r[q] = (m >> (d > 0 ? d : 0)) + (rest > half) + (q ? r[q - 1] : 0);
-            if (d < 2 || rest == half) odd |= 1u << q;
+            if (d < 2 || rest == half || b < 0) odd |= 1u << q;
         }
         long long sum = r[3];
 #pragma unroll
