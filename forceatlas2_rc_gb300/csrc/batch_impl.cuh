@@ -99,10 +99,10 @@ template <int W, int H> __device__ double block_sum(const double (&v)[H], double
     return __dadd_rn(s, c);
 }
 
-// Two sums over the block of V threads' values each (H a thread), added in pairs:
-// by warp, then the V / 32 warps' sums by a warp each. Into a[0] and b[0]. Warps
-// that hold none of the n values have 0 and add nothing up (an FP64 instruction
-// of a warp takes the SM 16 cycles).
+// Two sums over the block of V threads' values each (H a thread): by warp, added
+// in pairs, then the V / 32 warps' sums by a warp each, rounded once
+// (warp_sum_once). Into a[0] and b[0]. Warps that hold none of the n values have
+// 0 and add nothing up (an FP64 instruction of a warp takes the SM 16 cycles).
 template <int W, int H>
 __device__ void block_sums(int n, const double (&x)[H], const double (&y)[H], double *a, double *b)
 {
@@ -123,7 +123,7 @@ __device__ void block_sums(int n, const double (&x)[H], const double (&y)[H], do
     __syncthreads();
     if (w < 2) {
         double *v = w == 0 ? a : b;
-        const double sum = warp_sum(v[lane]);
+        const double sum = warp_sum_once(v[lane]);
         __syncwarp();
         if (lane == 0) v[0] = sum;
     }
@@ -512,8 +512,8 @@ k_batch(int ngraphs, BatchGraph *graphs, const int *queue, int *next, int iterat
             }
             double tsw, ttr;
             if constexpr (sizeof(R) == 4) {
-                // both at once, by pairs to the end (a serial sum over the
-                // warps, compensated, took 100 dependent FP64 operations)
+                // both at once (a serial sum over the warps, compensated, took
+                // 100 dependent FP64 operations)
                 block_sums<W>(n, ts, tt, red, red2);
                 tsw = red[0];
                 ttr = red2[0];
