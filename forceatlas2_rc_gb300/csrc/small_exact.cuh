@@ -19,6 +19,7 @@ namespace fa2cu {
 // barriers, two dependent FP64 divisions of the speed update), from 1,000 nodes
 // by the pairs on 16 of the SMs.
 constexpr int SE_THREADS = 512;
+static_assert(CS_MAX_BLOCKS == 16, "half a warp holds the blocks' sums");
 constexpr int SE_MAX = 1500; // nodes up to which it is the faster
 constexpr int SE_PARTS = 16; // of the sources, at most
 constexpr int SE_ITERATIONS = 256; // a launch, at most
@@ -60,6 +61,7 @@ k_small_exact(int n, int m, int iterations, float scaling, float gravity, int st
     __shared__ float4 warp_sum4[T / 32], block_sum4[CS_MAX_BLOCKS];
     __shared__ SpeedState speed;
     __shared__ int stop;
+    __shared__ double traction;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned rank = blockIdx.x, blocks = gridDim.x; // one cluster
     const int base = (int) rank * m, cnt = max(0, min(m, n - base));
@@ -155,14 +157,22 @@ k_small_exact(int n, int m, int iterations, float scaling, float gravity, int st
         }
         if (blocks > 1) cluster_barrier();
         else __syncthreads();
+        // the blocks' sums (hi, lo), a lane each, rounded once: the swinging's by
+        // the first warp, the traction's by the second
+        double a = 0.0;
+        if (w < 2 && blocks > 1) {
+            const float4 v = (lane & 15) < (int) blocks ? block_sum4[lane & 15]
+                                                        : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            a = warp_sum_once((double) (lane < 16 ? w ? v.z : v.x : w ? v.w : v.y));
+            if (w == 1 && lane == 0) traction = a;
+            asm volatile("bar.sync 1, 64;" ::: "memory");
+        }
         if (w == 0) {
-            const float4 v = lane < (int) blocks ? block_sum4[lane]
-                                                 : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            double a = (double) v.x + (double) v.y, b = (double) v.z + (double) v.w;
-            for (int o = CS_MAX_BLOCKS / 2; o > 0; o >>= 1) {
-                if (o >= (int) blocks) continue;
-                a = __dadd_rn(a, __shfl_down_sync(0xffffffffu, a, o));
-                b = __dadd_rn(b, __shfl_down_sync(0xffffffffu, b, o));
+            double b = traction;
+            if (blocks == 1) {
+                const float4 v = block_sum4[0];
+                a = (double) v.x + (double) v.y;
+                b = (double) v.z + (double) v.w;
             }
             if (lane == 0) {
                 if (!(a == a) || !(b == b)) {
