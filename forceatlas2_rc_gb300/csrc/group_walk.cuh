@@ -410,9 +410,10 @@ __device__ __forceinline__ void group_top(GroupTopShared &T, GroupWalkShared &S,
         __syncwarp();
     }
     if (lane == 0) {
-        if (nfar & 1) { // an unused place: no mass, at a finite distance
+        if (nfar & 1) { // an unused place: no mass, far where the one beside it is
             GroupPair &p = T.far[nfar >> 1];
-            p.x[1] = p.y[1] = 1e18f;
+            p.x[1] = p.x[0];
+            p.y[1] = p.y[0];
             p.m[1] = 0.0f;
         }
         T.nfar = (nfar + 1) & ~1;
@@ -487,7 +488,8 @@ __device__ __forceinline__ void group_walk(const GroupTopShared &T, GroupWalkSha
             }
         }
         // the far regions first, then the mixed ones, each from an even
-        // place; the place left over by an odd count has no mass and no lanes
+        // place; the place left over by an odd count has no mass and no lanes,
+        // that of the far ones the last one's place (at a distance from all nodes)
         const unsigned wb = __ballot_sync(FULL, verdict == 1), mb = __ballot_sync(FULL, verdict == 0);
         const int nw = __popc(wb), nm = __popc(mb), m0 = (nw + 1) & ~1, end = m0 + nm;
         const int at = verdict == 1 ? __popc(wb & below) : m0 + __popc(mb & below);
@@ -500,9 +502,10 @@ __device__ __forceinline__ void group_walk(const GroupTopShared &T, GroupWalkSha
             p.floor[at & 1] = floor;
             p.lanes[at & 1] = lanes;
         }
-        if (lane == 0 && (nw & 1)) {
-            GroupPair &p = S.entry[nw >> 1];
-            p.x[1] = p.y[1] = 1e18f;
+        if (verdict == 1 && at == nw - 1 && (nw & 1)) {
+            GroupPair &p = S.entry[at >> 1];
+            p.x[1] = -c.x;
+            p.y[1] = -c.y;
             p.m[1] = 0.0f;
         }
         if (lane == 0 && (nm & 1)) {
