@@ -462,6 +462,10 @@ k_codes_sort(int n, int m, const typename RT<R>::R2 *__restrict__ pos,
 {
     constexpr int WARPS = T / 32, PARTS = T / 256; // threads a digit, eight warps each
     extern __shared__ __align__(16) uint2 cs_pairs[];
+    __shared__ uint32_t wh[WARPS][256];              // a warp's counts, then their prefix
+    __shared__ uint32_t table[2][CS_MAX_BLOCKS][256];   // the blocks' counts, by pass parity
+    __shared__ uint32_t lbase[256], gbase[256];
+    __shared__ uint2 wt[8];
     // bytes of the counts, and of the pairs, that arrive in a pass: a phase of
     // bar_pairs a pass, of bar_counts every other pass (cs_count_bar).
     // Counts: a block X sends those of pass p + 1 when it holds those of pass p
@@ -473,11 +477,9 @@ k_codes_sort(int n, int m, const typename RT<R>::R2 *__restrict__ pos,
     // Pairs: X sends those of pass p when it holds the counts of p of every Y,
     // which Y sent after its phase of the pairs of p - 1 and its last reads of
     // the array that the pairs of p go to.
+    // (Behind the arrays: before them, three words shift these off 16 bytes, which
+    // cost 1 to 2 us an iteration.)
     __shared__ uint64_t bar_counts[CS_COUNT_BARS], bar_pairs;
-    __shared__ uint32_t wh[WARPS][256];              // a warp's counts, then their prefix
-    __shared__ uint32_t table[2][CS_MAX_BLOCKS][256];   // the blocks' counts, by pass parity
-    __shared__ uint32_t lbase[256], gbase[256];
-    __shared__ uint2 wt[8];
     const unsigned rank = blockIdx.x, blocks = gridDim.x; // one cluster
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int base = (int) rank * m, cnt = max(0, min(m, n - base));
