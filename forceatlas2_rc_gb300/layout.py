@@ -75,9 +75,11 @@ def _flag(x, name):
 
 
 def _edges(n, edges):
-    e = np.asarray(edges if edges is not None else np.zeros((0, 2)))
-    if e.dtype.kind not in "iu":
-        e = e.astype(np.int64)
+    if edges is None:
+        edges = np.zeros((0, 2), np.int64)
+    e = np.asarray(edges)
+    if e.dtype.kind not in "iu":  # (from the argument: a list's values are checked one by one)
+        e = np.asarray(edges, dtype=np.int64)
     if e.size == 0:
         return np.zeros(0, np.int32), np.zeros(0, np.int32)
     if e.ndim != 2 or e.shape[1] != 2:
@@ -94,11 +96,14 @@ def _edges(n, edges):
 def edge_weights(m, weights, edge_weight_influence=1.0, normalize_weights=False,
                  invert_weights=False):
     """Weights as the package transforms them (R/forceatlas2.R:254-264)."""
+    invert_weights, normalize_weights = bool(invert_weights), bool(normalize_weights)
     if weights is None:
-        return np.ones(m)  # which every transformation leaves as they are
+        w = np.ones(m)
+        if isinstance(edge_weight_influence, (int, float)):
+            return w  # which every transformation leaves as they are
     else:
         try:
-            w = np.asarray(weights, dtype=np.float64).reshape(-1)
+            w = np.array(weights, dtype=np.float64).reshape(-1)  # (the result is a copy)
         except (TypeError, ValueError):
             raise ValueError("`weights` must be a numeric vector with one value "
                              f"per edge ({m}).") from None
