@@ -96,9 +96,9 @@ def _edges(n, edges):
 def edge_weights(m, weights, edge_weight_influence=1.0, normalize_weights=False,
                  invert_weights=False):
     """Weights as the package transforms them (R/forceatlas2.R:254-264)."""
-    invert_weights, normalize_weights = bool(invert_weights), bool(normalize_weights)
     if weights is None:
         w = np.ones(m)
+        invert_weights, normalize_weights = bool(invert_weights), bool(normalize_weights)
         if isinstance(edge_weight_influence, (int, float)):
             return w  # which every transformation leaves as they are
     else:
