@@ -1,9 +1,10 @@
 // batch_impl.cuh -- many independent layouts in one persistent launch.
 // Included by inst_f32.cu and inst_f64.cu only.
 //
-// Each graph of a batch is laid out by one thread block from start to end:
-// the block takes the next graph from a work counter (largest first), then
-// runs every step of every requested iteration for it:
+// Each graph of a batch is laid out by one thread block from start to end (in
+// FP32 one of 1,024 threads, in a launch of its own, if it would outlast the
+// others): the block takes the next graph from a work counter (largest first),
+// then runs every step of every requested iteration for it:
 //   - bounding box;
 //   - Morton codes;
 //   - a block-level stable radix sort;
@@ -14,8 +15,11 @@
 //   - the swing/traction totals reduced by the block, the FP64 speed update
 //     of that graph;
 //   - the displacement.
-// No block ever waits for another, and a graph's result depends on nothing
-// but the graph and the block size: it is the same alone or in any mix.
+// No block waits for another while it has work. The blocks of the second launch
+// wait at their end for the first launch's (griddepcontrol.wait), which cannot
+// depend on them: every block of the first is on an SM before the second starts.
+// A graph's result depends on nothing but the graph and the batch's block size,
+// and not on which launch had it: it is the same alone or in any mix.
 //
 // Device arrays are the concatenation of the graphs' arrays (node arrays at
 // the graph's first node, its incidences at its first incidence, node indices
@@ -271,8 +275,9 @@ __device__ __forceinline__ void block_exact_tiles(int n, bool two, R scaling,
 
 // FP32: two blocks of 512 (four of 256) threads per SM, 64 registers a thread,
 // which the group walk wants (three blocks at 40 registers: 3.01 against 2.85
-// ms an iteration of 1,024 graphs of 50 to 20,000 nodes). FP64 needs more
-// registers: one block of 512 (two of 256).
+// ms an iteration of 1,024 graphs of 50 to 20,000 nodes, which lasted as long as
+// its largest graph; the walk's arrays of three, 76 KB each, do not fit an SM).
+// FP64 needs more registers: one block of 512 (two of 256).
 // FP32 graphs that would outlast the others (wide_graphs) are taken by blocks
 // of WIDE threads, which have an SM each. They are launched first, and the
 // other blocks when all of them have started (launch_kernel).

@@ -120,8 +120,6 @@ enum {
     ERR_BOUNDS = 4,    // a computed index or walk left its bounds (a bug)
 };
 
-// Speed-controller state on the device, in double (reference
-// src/forceatlas2.c:445-485 runs it on the host; here it never leaves HBM).
 // What the speed update needs of the number of nodes, made once a layout (the
 // two square roots took the totals' last thread about 2 us an iteration).
 struct SpeedTerms {
@@ -135,6 +133,8 @@ inline __host__ __device__ SpeedTerms speed_terms(int n)
     t.n2 = (double) n * (double) n;
     return t;
 }
+// Speed-controller state on the device, in double (reference
+// src/forceatlas2.c:445-485 runs it on the host; here it never leaves HBM).
 struct SpeedState {
     double speed, efficiency;
     double total_swinging, total_traction;

@@ -2361,7 +2361,7 @@ k_pack_exact(int n, const double *__restrict__ x, const double *__restrict__ y,
 //
 // Bound: the FP32 pipe, 7 operations a pair (and one MUFU reciprocal, at half
 // their time); the packed instructions leave its issue slots for the rest.
-// 100,003 nodes: 2906 -> 2426 us (77 % of the pipe at 2070 MHz; with 4 nodes a
+// 100,003 nodes: 2906 -> 2428 us (the pipe 74 % busy; with 4 nodes a
 // thread 2568, with 8 2525, with 10 2471).
 
 constexpr int EXACT_THREADS = 256;

@@ -13,7 +13,7 @@ namespace fa2cu {
 //
 // Why: three launches an iteration took 15 to 20 us for a few of arithmetic. An
 // iteration in us, three launches and this with 1 / 4 / 16 blocks: 50 nodes
-// 15.0 and 4.3 / 5.2 / 5.5; 150 14.9 and 5.5 (now 5.3) / 6.2 / 6.3; 300 15.9 and 9.7 /
+// 15.0 and 4.3 / 5.2 / 5.5; 150 14.9 and 5.5 (now 5.1) / 6.2 / 6.3; 300 15.9 and 9.7 /
 // 7.6 / 7.3; 1,000 18.2 and - / 20.0 / 11.3; 1,500 19.8 and - / 39.2 / 16.6;
 // 2,000 21.1 and - / 59.9 / 22.6. Bound by latency (the block's and cluster's
 // barriers, two dependent FP64 divisions of the speed update), from 1,000 nodes

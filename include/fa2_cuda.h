@@ -122,9 +122,10 @@ int fa2cu_layout_traversal_counts(fa2cu_layout *L, double counts[2]);
  *                  equal to ~1e-7);
  *   "attract_grid" blocks per SM of that attraction, 1 to 8 (default 1, 2
  *                  above 110,000 nodes);
- *   "join_blocks"  blocks of 256 threads of the join that adds it to the
- *                  repulsion and sums the swing totals (default 608: few
- *                  block partials for its last block);
+ *   "join_blocks"  blocks of the join that adds it to the repulsion and sums
+ *                  the swing totals, at most (of 64 threads below 20,000
+ *                  nodes, 128 below 200,000, else 256; default 608: few block
+ *                  partials for its last block);
  *   "pdl"          1: the iteration's kernels on the main stream launched
  *                  as programmatic dependents (each is scheduled as its
  *                  predecessor finishes; default below 500,000 nodes), 0:
