@@ -787,15 +787,23 @@ __device__ __forceinline__ double4_32a agg_record(const Agg<double> &q, double /
 // In float, the record holds w = size^2 * wscale with wscale = (1 + B) /
 // theta^2 (B = DECIDE_BAND): the walk's opening test is then d^2 > w, with
 // the band of decisions made again in double right below it (region_far).
+// A rounded centre of mass that its rounding (at most 2 units) put outside the
+// box is moved to the edge. One farther out stays: masses of both signs have it
+// there; no number (no mass in all) stays none, and its region is opened.
+__device__ __forceinline__ float box_centre(float c, float lo, float hi)
+{
+    const float most = 4.76837158203125e-07f * fmaxf(fabsf(lo), fabsf(hi)); // 2^-21
+    if (c < lo && lo - c <= most) return lo;
+    return c > hi && c - hi <= most ? hi : c;
+}
 __device__ __forceinline__ float4 agg_record(const Agg<float> &q, float wscale)
 {
     const float m = q.m.hi + q.m.lo;
     const float w = q.maxx - q.minx, h = q.maxy - q.miny;
-    // the rounded centre kept inside the box: a region of coincident nodes (w
-    // = h = 0) has its centre exactly at its nodes, which are then not far
-    // from it
-    const float cx = fminf(fmaxf(__fdiv_rn(q.mx.hi + q.mx.lo, m), q.minx), q.maxx);
-    const float cy = fminf(fmaxf(__fdiv_rn(q.my.hi + q.my.lo, m), q.miny), q.maxy);
+    // a region of coincident nodes (w = h = 0) has its centre exactly at its
+    // nodes, which are then not far from it
+    const float cx = box_centre(__fdiv_rn(q.mx.hi + q.mx.lo, m), q.minx, q.maxx);
+    const float cy = box_centre(__fdiv_rn(q.my.hi + q.my.lo, m), q.miny, q.maxy);
     return make_float4(cx, cy, m, 2.0f * (w * w + h * h) * wscale);
 }
 
